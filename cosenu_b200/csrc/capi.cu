@@ -488,17 +488,17 @@ int ctx_create(const cosenu_params *pp, cosenu_ctx **out, int layout)
     if (ctx->use_tma) {
         // box rows follow the row count of the stages that read each map (the TMA
         // kernel's rows(): 12 for the latency-bound FD stages, else 8)
-        const int ub = ctx->fp32 ? 4 : 8, bx = tma_box_x(8), bxu = tma_box_x(ub),
-                  bt = tma_box_tile(), rw = tma_box_rows(p.scheme, true),
+        const int ub = ctx->fp32 ? 4 : 8, bx = tma_box_x(p.scheme, 8, false),
+                  bxu = tma_box_x(p.scheme, ub, false), bt = tma_box_tile(), rw = tma_box_rows(p.scheme, true),
                   rn = tma_box_rows(p.scheme, false), ru = ctx->fp32 ? rw : rn;
         int r = make_state_map(&ctx->mYb40[0], ctx->Yb[0], 8, ctx->ld, p.nvz, ctx->cs, bx, rw);
         if (!r) r = make_state_map(&ctx->mYb40[1], ctx->Yb[1], 8, ctx->ld, p.nvz, ctx->cs, bx, rw);
         if (!r) r = make_state_map(&ctx->mYb40s4[0], ctx->Yb[0], 8, ctx->ld, p.nvz, ctx->cs, bx, rn);
         if (!r) r = make_state_map(&ctx->mYb40s4[1], ctx->Yb[1], 8, ctx->ld, p.nvz, ctx->cs, bx, rn);
         if (!r) r = make_state_map(&ctx->mU0_40, ctx->U0, ub, ctx->ld, p.nvz, ctx->cs, bxu, ru);
-        // (FP64 stage 3 reads U1 in 40-cell rows, see the TMA kernel's Layout)
+        // (the input box of FP64 stage 3)
         if (!r) r = make_state_map(&ctx->mU1_40, ctx->U1, ub, ctx->ld, p.nvz, ctx->cs,
-                                   ctx->fp32 ? bxu : bt + 8, ru);
+                                   tma_box_x(p.scheme, ub, !ctx->fp32), ru);
         if (!r) r = make_state_map(&ctx->mY32, ctx->Yb[0], 8, ctx->ld, p.nvz, ctx->cs, bt, rn);
         if (!r) r = make_state_map(&ctx->mA32, ctx->Yb[1], 8, ctx->ld, p.nvz, ctx->cs, bt, rn);
         if (!r) r = make_state_map(&ctx->mU0_32, ctx->U0, ub, ctx->ld, p.nvz, ctx->cs, bt, rn);

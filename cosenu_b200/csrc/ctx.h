@@ -20,7 +20,7 @@ cudaError_t launch_moments(const double *X, double *M, const double *vz, long lo
 int make_state_map(CUtensorMap *map, const void *base, int elem_bytes, int ld, int nvz,
                    long long cs, int box_cells, int box_rows);
 int tma_box_rows(int scheme, bool wide);
-int tma_box_x(int elem_bytes);
+int tma_box_x(int scheme, int elem_bytes, bool narrow);
 int tma_box_tile();
 int tma_max_nvz();
 int tma_blocks_per_sm(int scheme);

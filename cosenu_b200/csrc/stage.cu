@@ -64,25 +64,26 @@ __device__ __forceinline__ double face_at(const TIN *__restrict__ X, const doubl
     if constexpr (INC) {
         // stencil differences as (Y difference in FP64, rounded) + (D
         // difference in FP32); the face is Y + (D + correction)
-        float d[7];
+        float dl[6];
         const double y0 = YPLUS ? ld_nc(Y + i) : (double)ld_nc(X + i);
         const float x0 = YPLUS ? (float)ld_nc(X + i) : 0.f;
 #pragma unroll
-        for (int k = -3; k <= 3; ++k) {
-            if (k == 0) continue;
-            const long long j = i + k * dir;
+        for (int k = 0; k < 6; ++k) {
+            const long long j0 = i + (k - 3) * dir, j1 = i + (k - 2) * dir;
             if constexpr (YPLUS)
-                d[k + 3] = (float)(ld_nc(Y + j) - y0) + ((float)ld_nc(X + j) - x0);
+                dl[k] = (float)(ld_nc(Y + j1) - ld_nc(Y + j0)) +
+                        ((float)ld_nc(X + j1) - (float)ld_nc(X + j0));
             else
-                d[k + 3] = (float)((double)ld_nc(X + j) - y0);
+                dl[k] = (float)((double)ld_nc(X + j1) - (double)ld_nc(X + j0));
         }
-        const float corr = weno7_corr(d[0], d[1], d[2], d[4], d[5], d[6]);
-        return y0 + (double)(x0 + corr);
+        return y0 + (double)(x0 + weno7_corr12(dl) * (1.f / 12.f));
     } else {
-        double u[7];
+        double u[7], dl[6];
 #pragma unroll
         for (int k = -3; k <= 3; ++k) u[k + 3] = in_at<YPLUS>(X, Y, i + k * dir);
-        return weno7_face(u[0], u[1], u[2], u[3], u[4], u[5], u[6]);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) dl[k] = u[k + 1] - u[k];
+        return u[3] + weno7_corr12(dl) * (1.0 / 12.0);
     }
 }
 

@@ -1,183 +1,58 @@
-// TMA-pipelined RK4 stage kernel for the FV (src/rhs_fv.hpp:115-236) and FD
-// (src/rhs_fd.hpp:6-148) schemes.
+// TMA-pipelined RK4 stage kernel of the FD scheme (src/rhs_fd.hpp:6-148); the
+// FV scheme's is stage_fv.cu.
 //
 // Same arithmetic and epilogue as rk4_stage_kernel (stage.cu); what changes
 // is how the operands reach the SM.  Each block is persistent over z-tiles of
-// 32 cells that span all nvz rows.  One producer warp streams chunks of 8 rows
-// x (32 + 2*4) cells of all 8 components of the stage input, and the matching
-// 8 x 32 cells of Y and A, into a ring of NBUF shared-memory buffers with
+// 32 cells that span all nvz rows.  One producer warp streams chunks of 8 (or
+// 12) rows x (32 + 2*4) cells of all 8 components of the stage input, and the
+// matching cells of Y and A, into a ring of NBUF shared-memory buffers with
 // cp.async.bulk.tensor (one 3-D tensor-map copy per operand and chunk, box
-// {cells, rows, components}); eight consumer warps take one row each, read
+// {cells, components, rows}); the consumer warps take one row each, read
 // their stencil from shared memory and write the results with coalesced
 // stores.  Full/empty mbarriers order the ring.  With up to NBUF-1 chunks in
 // flight (~100 KB per SM) the kernel keeps HBM busy without depending on
-// occupancy, which the register-heavy FP64 right-hand side limits.  FD runs
-// one block per SM; FV, bound by FP64 issue rather than HBM, runs two (each
-// with half the shared memory) so that twice the warps hide the latency of the
-// WENO7 arithmetic.  FV launches have no producer warp: the last consumer
-// warp to release a buffer issues its next copies, so a block is 8 warps and
-// gets 128 registers per thread.  Per-row velocities and
-// advection factors equal the host's tables (src/nuosc.hpp:88-92,
-// rhs_fv.hpp:145, rhs_fd.hpp:57): FV reads them once per chunk through the
-// read-only cache, FD recomputes them in registers.
+// occupancy, which the register-heavy FP64 right-hand side limits.  One block
+// per SM.  Per-row velocities and advection factors equal the host's tables
+// (src/nuosc.hpp:88-92, rhs_fd.hpp:57) and are recomputed in registers.
 //
-// FV: a warp holds one row, so every lane reconstructs the upwind WENO7 face it
-// owns from the shared-memory stencil and takes its neighbour's face by
-// shuffle; the one face per row and component outside the tile is computed,
-// for all rows of a chunk at once, by R*8/32 warps in turn and published in
-// shared memory (Layout::NE).  FD: the common variant of manage.py (central
-// FD4 + KO3) is a compile-time fast path; the upwind / lopsided / KO5 variants
-// take the generic path.
+// The common variant of manage.py (central FD4 + KO3) is a compile-time fast
+// path; the upwind / lopsided / KO5 variants take the generic path.
 //
 // Every wait is bounded in time (globaltimer, limit StageArgs::wait_ns): on
 // expiry the kernel records a code in *err and carries on along the same
 // control path, so no barrier is left waiting and the host reports the error.
 // After a failed wait a consumer warp does not release its buffer, so the
-// producer's next wait on that buffer fails too and it stops issuing copies
-// (without a producer warp the buffer's release count never completes and no
-// warp refills it); before the block exits one thread waits (bounded again)
-// for the copies in flight, so no block ends while a bulk copy still writes
-// into its shared memory.
-#include <cuda.h>
+// producer's next wait on that buffer fails too and it stops issuing copies;
+// before the block exits it waits (bounded again) for the copies in flight, so
+// no block ends while a bulk copy still writes into its shared memory.
+#include <cstdlib>
 
-#include <type_traits>
-
-#include "common.cuh"
-#include "weno.cuh"
+#include "tma.cuh"
 
 namespace cosenu {
 
 namespace tma {
 
-constexpr int TZ = 32;           // cells per tile (one warp lane each)
-constexpr int HALO = 4;          // cells each side in the input box
 // Width of an input box row: the tile plus HALO cells each side, rounded up so
-// that the row is a multiple of 16 bytes (TMA) and the component rows of one
-// v row start in distinct shared-memory banks: the edge faces of a row read
-// the same cell of all 8 components at once (42 doubles = 84 words: banks
-// 0, 20, 8, 28, ... for components 0..7; 44 floats = 44 words: 0, 12, 24, ...).
+// that the row is a multiple of 16 bytes (TMA).
 template <class T> constexpr int xw() { return sizeof(T) == 8 ? 42 : 44; }
-// v rows per chunk = consumer warps.  FV runs two blocks per SM with 8.  FD runs one block per SM: the stages that move
-// few bytes per cell (FP64 stage 1, FP32-bulk stages 1-3) are bound by latency
-// and run 12 (13 warps, ~126 registers, no spills: 0.230 -> 0.205 ms for FP64
-// stage 1 at nz 32768 x nvz 256); the HBM-bound stages keep 8, whose smaller
-// chunks keep fewer bytes in flight (12 rows: FP64 stage 3 0.436 -> 0.490 ms).
-template <int SCHEME, int STAGE, bool INC> constexpr int rows()
+// v rows per chunk = consumer warps.  The stages that move few bytes per cell
+// (FP64 stage 1, FP32-bulk stages 1-3) are bound by latency and run 12 (13
+// warps, ~126 registers, no spills: 0.230 -> 0.205 ms for FP64 stage 1 at nz
+// 32768 x nvz 256); the HBM-bound stages keep 8, whose smaller chunks keep
+// fewer bytes in flight (12 rows: FP64 stage 3 0.436 -> 0.490 ms).
+template <int STAGE, bool INC> constexpr int rows()
 {
-    return (SCHEME == FD && ((!INC && STAGE == 1) || (INC && STAGE <= 3))) ? 12 : 8;
-}
-// tensor maps per ensemble member (MapIdx lists them)
-constexpr int NMAP = 8;
-#define TMA_MAX_NVZ 1024
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ unsigned long long gtimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Bounded wait; returns false (and records `code`) when `limit_ns` passes.
-// Once any wait in the grid has expired (*err != 0) later waits give up
-// at once, so a broken pipeline ends within one time limit.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err, int code,
-                                          unsigned long long limit_ns)
-{
-    if (mbar_try(bar, parity)) return true;
-    volatile int *verr = err;
-    if (*verr != 0) return false;
-    const unsigned long long t0 = gtimer();
-    for (uint32_t n = 1;; ++n) {
-        if (mbar_try(bar, parity)) return true;
-        if ((n & 63) == 0 && (*verr != 0 || gtimer() - t0 > limit_ns)) {
-            atomicCAS(err, 0, code);
-            return false;
-        }
-    }
-}
-
-// Wait for the completion of copies already issued, whatever *err says
-// (bounded by `limit_ns`, code 3 on expiry): the producer's last act.
-__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity, int *err,
-                                           unsigned long long limit_ns)
-{
-    if (mbar_try(bar, parity)) return;
-    const unsigned long long t0 = gtimer();
-    for (uint32_t n = 1;; ++n) {
-        if (mbar_try(bar, parity)) return;
-        if ((n & 63) == 0 && gtimer() - t0 > limit_ns) {
-            atomicCAS(err, 0, 3);
-            return;
-        }
-    }
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(
-                     smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z,
-                                            uint64_t *bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-        "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Brings a tensor map held in global memory into the TMA unit's cache.
-__device__ __forceinline__ void prefetch_map(const CUtensorMap *map)
-{
-    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
-}
-
-template <int NCONS> __device__ __forceinline__ void consumer_sync()
-{
-    asm volatile("bar.sync 1, %0;" ::"n"(NCONS) : "memory");
+    return ((!INC && STAGE == 1) || (INC && STAGE <= 3)) ? 12 : 8;
 }
 
 // One ring buffer holds, for R rows, boxes laid out [row][component][cell]
 // (the tensor maps put components before rows): the input box X, then Y, then
 // the own-cell tiles A (and B).
-template <int SCHEME, class TIN, class TOUT, int STAGE> struct Layout {
+template <class TIN, class TOUT, int STAGE> struct Layout {
     static constexpr bool INC = inc_form<TIN, TOUT>();
-    static constexpr int R = rows<SCHEME, STAGE, INC>();
+    static constexpr int R = rows<STAGE, INC>();
     static constexpr int NTHR = R * 32 + 32;  // consumer warps + producer warp
-    // without a producer warp (see producer_warp)
-    static constexpr int NTHR_NP = R * 32;
     // FP64 stage 3 streams the most bytes per chunk: its 40-cell rows keep a
     // two-buffer ring within half an SM's shared memory (two blocks per SM)
     static constexpr int XW = (!INC && STAGE == 3) ? TZ + 2 * HALO : xw<TIN>();
@@ -192,50 +67,9 @@ template <int SCHEME, class TIN, class TOUT, int STAGE> struct Layout {
     static constexpr int AB = INC ? (STAGE == 4 ? 2 * NCOMP * R * TZ * 4 : 0)
                                   : (STAGE >= 3 ? NCOMP * R * TZ * 8 : 0);
     static constexpr int BUF = ((XB + YB + AB) + 127) / 128 * 128;
-    // FV (two blocks per SM, 96-128 registers): each consumer warp accumulates
-    // the output moments of its rows in shared memory rather than in 12
-    // registers, where half an SM leaves room (all but FP64 stage 3); the
-    // other kernels keep them in registers and pair warps at the tile's end
-    static constexpr bool MSM = SCHEME == FV && (INC || STAGE != 3);
-    static constexpr int NRED = MSM ? R : R / 2;  // moment slots in shared memory
-    // FV: the face of each row and component at the tile's upwind edge lies
-    // outside the warp's 32 lanes.  Each chunk, NE = R * NCOMP / 32 warps (in
-    // turn) compute all of them at full lane occupancy and publish them in
-    // shared memory (one slot array and one mbarrier per ring buffer), rather
-    // than every warp spending a ninth WENO7 pass with 8 of 32 lanes active.
-    static constexpr int NE = SCHEME == FV ? R * NCOMP / 32 : 0;
-    static_assert(NE == 0 || (R * NCOMP % 32 == 0 && (R & (R - 1)) == 0),
-                  "edge warps: whole warps, rows a power of two");
+    // output moments: registers per warp, paired at the tile's end
+    static constexpr int NRED = R / 2;  // moment slots in shared memory
 };
-
-// FD launches stream through a producer warp.  FV launches (single
-// simulations and ensembles) run without one: the last consumer warp to
-// release a ring buffer issues that buffer's next copies itself.  Its block is
-// then 8 warps, and two blocks per SM get 128 registers per thread instead of
-// the 96 that two 9-warp blocks leave (FP64 stage 3 spilled at 96).
-template <int SCHEME, bool BATCHED> __host__ __device__ constexpr bool producer_warp()
-{
-    return SCHEME == FD;
-}
-
-// Arrival counter of a ring buffer without a producer warp: acquire-release
-// add, so the last warp's refill is ordered after every warp's reads.
-__device__ __forceinline__ uint32_t ring_release_count(uint32_t *cnt)
-{
-    uint32_t old;
-    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
-                 : "=r"(old)
-                 : "r"(smem_u32(cnt))
-                 : "memory");
-    return old;
-}
-
-// Orders this thread's generic-proxy view of shared memory before the bulk
-// copies it issues next.
-__device__ __forceinline__ void fence_proxy_async_smem()
-{
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 
 // The copies of one ring buffer: the stage input box (X) and, where the
 // stage reads them, Y and the own-cell tiles A (and B), all completing on
@@ -255,39 +89,12 @@ __device__ __forceinline__ void issue_chunk(unsigned char *buf, uint64_t *bar, c
     }
 }
 
-// Index of each operand's tensor map among a member's NMAP maps (ensembles).
-// FP64:      0 Y (halo box), 1 U0 (halo), 2 U1 (halo), 3 Y (tile), 4 A (tile), 5 U0 (tile)
-// FP32-bulk: 0 current Y (halo), 1 D1 (halo), 2 D2 (halo), 3 D2 (tile), 5 D1 (tile), 6 D3 (halo),
-//            7 current Y (halo) in the row count of stage 4
-template <bool INC, int STAGE> struct MapIdx {
-    static constexpr int X = STAGE == 1 ? 0 : (STAGE == 3 ? 2 : (INC && STAGE == 4 ? 6 : 1));
-    static constexpr int Y = INC ? (STAGE == 4 ? 7 : 0) : 3;
-    static constexpr int A = INC ? 5 : (STAGE == 3 ? 5 : 4);
-    static constexpr int B = 3;
-};
-
 }  // namespace tma
-
-static_assert(sizeof(StageArgs) % 8 == 0, "StageArgs is copied to shared memory in 8-byte words");
-
-template <bool BATCHED>
-__device__ __forceinline__ void tma_tile(const BatchDev &bd, int t, int &inst, int &zt)
-{
-    if (BATCHED) {
-        const int4 e = bd.table[t];
-        inst = e.x;
-        zt = e.y;
-    } else {
-        inst = 0;
-        zt = t;
-    }
-}
 
 // FD: velocity and advection factor of row i, recomputed with round-to-nearest
 // operations so the bits equal the host tables (capi.cu, src/nuosc.hpp:88-92,
 // rhs_fd.hpp:57).  The FD stages are bound by memory latency, and a table load
-// per chunk slowed them (FP64 stages 1, 2, 4 at nz 32768 x nvz 256 by 8 %); the
-// FP64-bound FV stages read the tables instead.
+// per chunk slowed them (FP64 stages 1, 2, 4 at nz 32768 x nvz 256 by 8 %).
 __device__ __forceinline__ void fd_row_values(double v0, double dv, double dz, int fd_advec, int i,
                                               double &v, double &f)
 {
@@ -302,13 +109,9 @@ __device__ __forceinline__ void fd_row_values(double v0, double dv, double dz, i
 // TIN: type of the streamed stage input (FP64: the stage value U or Y;
 // FP32-bulk: Y at stage 1, the increment D after).  TOUT: type of the output
 // (FP64: U', U'' or Y; FP32-bulk: D1, D2, D3, then the new Y).  The
-// right-hand side is evaluated in FP64 in both forms, except the FP32-bulk
-// WENO7 weights and candidates (FP32 on FP64 stencil differences).
-template <int SCHEME, bool GEN, int STAGE, class TIN, class TOUT, int NBUF, bool BATCHED, int MINB>
-__global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
-                                      ? tma::Layout<SCHEME, TIN, TOUT, STAGE>::NTHR
-                                      : tma::Layout<SCHEME, TIN, TOUT, STAGE>::NTHR_NP,
-                                  MINB)
+// right-hand side is evaluated in FP64 in both forms.
+template <bool GEN, int STAGE, class TIN, class TOUT, int NBUF, bool BATCHED, int MINB>
+__global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
     rk4_stage_tma_kernel(const __grid_constant__ CUtensorMap mX,
                          const __grid_constant__ CUtensorMap mY,
                          const __grid_constant__ CUtensorMap mA,
@@ -316,7 +119,7 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
                          const __grid_constant__ StageArgs a0, int *err, const BatchDev bd)
 {
     using namespace tma;
-    using L = Layout<SCHEME, TIN, TOUT, STAGE>;
+    using L = Layout<TIN, TOUT, STAGE>;
     constexpr int R = L::R;
     auto consumer_sync = tma::consumer_sync<R * 32>;
     using MI = MapIdx<L::INC, STAGE>;
@@ -324,76 +127,22 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + NBUF * L::BUF);
     uint64_t *empty = full + NBUF;
-    uint64_t *ebar = empty + NBUF;  // FV: edge faces of buffer b published
-    double(*s_mom)[TZ] =
-        reinterpret_cast<double(*)[TZ]>(ebar + (L::NE ? NBUF : 0));  // [6][TZ]
+    double(*s_mom)[TZ] = reinterpret_cast<double(*)[TZ]>(empty + NBUF);  // [6][TZ]
     double(*s_red)[NMOM][TZ] = reinterpret_cast<double(*)[NMOM][TZ]>(s_mom + NMOM);  // [NRED]
     StageArgs *s_args = reinterpret_cast<StageArgs *>(s_red + L::NRED);  // batched: current member
-    // FV: [NBUF][R][NCOMP] edge faces
-    double(*s_edge)[R][NCOMP] = reinterpret_cast<double(*)[R][NCOMP]>(s_args + 1);
-    // without a producer warp: per ring buffer, the warps' release count and
-    // the last chunk whose copies went into it
-    constexpr bool PW = producer_warp<SCHEME, BATCHED>();
-    uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_edge + (L::NE ? NBUF : 0));
-    int *s_last = reinterpret_cast<int *>(s_cnt + NBUF);
-
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nzt = BATCHED ? bd.ntiles : a0.nz / TZ;
-    // without a producer warp: the block's chunks in order (its z tiles or
-    // table entries, each in chunks of R rows); chunk ch of tile t is the
-    // block's n-th chunk, and its copies go into buffer n % NBUF
-    const bool rr0 = !BATCHED || bd.range == nullptr;
-    const int te0 = rr0 ? nzt : bd.range[blockIdx.x + 1];
-    const int ts0 = rr0 ? gridDim.x : 1;
-    auto nch_of = [&](int t) { return ((BATCHED ? bd.table[t].w : a0.nvz) + R - 1) / R; };
-    auto issue_at = [&](int t, int ch, uint32_t n) {
-        if (a0.stall) return;
-        const int b = n % NBUF;
-        if constexpr (BATCHED) {
-            const int4 e = bd.table[t];
-            const CUtensorMap *m = &bd.maps[e.x * NMAP];
-            issue_chunk<L>(smem + b * L::BUF, &full[b], &m[MI::X], &m[MI::Y], &m[MI::A],
-                           &m[MI::B], e.y * TZ, ch * R);
-        } else {
-            issue_chunk<L>(smem + b * L::BUF, &full[b], &mX, &mY, &mA, &mB, t * TZ, ch * R);
-        }
-        s_last[b] = (int)n;
-    };
-    // (t, ch) moved k chunks on; false past the block's last tile
-    auto advance = [&](int &t, int &ch, int k) -> bool {
-        for (; k > 0; --k) {
-            if (++ch == nch_of(t)) {
-                ch = 0;
-                t += ts0;
-                if (t >= te0) return false;
-            }
-        }
-        return true;
-    };
 
     if (tid == 0) {
         for (int b = 0; b < NBUF; ++b) {
             tma::mbar_init(&full[b], 1);
             tma::mbar_init(&empty[b], R);
-            if (L::NE) tma::mbar_init(&ebar[b], L::NE * 32);
-            if constexpr (!PW) {
-                s_cnt[b] = 0;
-                s_last[b] = -1;
-            }
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if constexpr (!PW) {
-            int t = rr0 ? blockIdx.x : bd.range[blockIdx.x], ch = 0;
-            if (t < te0)
-                for (uint32_t n = 0; n < (uint32_t)NBUF; ++n) {
-                    issue_at(t, ch, n);
-                    if (!advance(t, ch, 1)) break;
-                }
-        }
     }
     __syncthreads();
 
-    if (PW && warp == R) {
+    if (warp == R) {
         // ------------------------------------------------------------ producer
         if (lane == 0 && !a0.stall) {
             uint32_t it = 0;
@@ -497,243 +246,82 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
                 mnext = an.Min[(long long)(tid / TZ) * an.nz + zn * TZ + tid % TZ];
         }
         double macc[NMOM] = {0, 0, 0, 0, 0, 0};
-        if constexpr (L::MSM) {
-            // this warp's moment slots (the previous tile's epilogue has read them)
-#pragma unroll
-            for (int m = 0; m < NMOM; ++m) s_red[warp][m][lane] = 0.0;
-        }
-
         for (int ch = 0; ch < nch; ++ch, ++it) {
             const int b = it % NBUF;
             const int v = ch * R + warp;
             const bool valid = v < a.nvz;
             const int vr = valid ? v : a.nvz - 1;
-            // the row's velocity and advection factor: FV from the host tables
-            // (read before the wait, so the load overlaps it), FD recomputed
             double vzv, factor;
-            if constexpr (SCHEME == FV) {
-                vzv = __ldg(&a.vz[vr]);
-                factor = __ldg(&a.rowfac[vr]);
-            } else {
-                fd_row_values(a.v0, a.dv, a.dz, a.fd_advec, vr, vzv, factor);
-            }
+            fd_row_values(a.v0, a.dv, a.dz, a.fd_advec, vr, vzv, factor);
             const bool landed = tma::mbar_wait(&full[b], (it / NBUF) & 1, err, 2, a0.wait_ns);
             const unsigned char *buf = smem + b * L::BUF;
-            // row r of component 0 in the input box (HALO cells each side); a
-            // row's components are XW cells apart
+            // this warp's row in the input boxes (HALO cells each side); a row's
+            // components are XW (YW) cells apart
             constexpr int XW = L::XW, YW = L::YW;
-            auto xrow_of = [&](int r) {
-                return reinterpret_cast<const TIN *>(buf) + r * (NCOMP * XW) + HALO;
-            };
-            auto yrow_of = [&](int r) {
-                return reinterpret_cast<const double *>(buf + L::XB) + r * (NCOMP * YW) +
-                       (INC ? HALO : 0);
-            };
-            const TIN *xrow = xrow_of(warp);  // this warp's row
-            const double *yrow = yrow_of(warp);
-            // the stage input at cell j of row x / y (j in [-HALO, TZ + HALO))
-            auto in_r = [&](const TIN *x, const double *y, int q, int j) -> double {
+            const TIN *xrow = reinterpret_cast<const TIN *>(buf) + warp * (NCOMP * XW) + HALO;
+            const double *yrow = reinterpret_cast<const double *>(buf + L::XB) +
+                                 warp * (NCOMP * YW) + (INC ? HALO : 0);
+            // the stage input at cell j of this row (j in [-HALO, TZ + HALO))
+            auto in = [&](int q, int j) -> double {
                 if constexpr (INC && STAGE >= 2)
-                    return y[q * YW + j] + (double)x[q * XW + j];
+                    return yrow[q * YW + j] + (double)xrow[q * XW + j];
                 else
-                    return (double)x[q * XW + j];
+                    return (double)xrow[q * XW + j];
             };
-            auto in = [&](int q, int j) -> double { return in_r(xrow, yrow, q, j); };
-            // FP32-bulk: the stencil difference u(j + k) - u(j) as
-            // (Y difference in FP64, rounded) + (D difference in FP32)
-            auto dif = [&](const TIN *x, const double *y, int q, int j, int k) -> float {
-                if constexpr (INC && STAGE >= 2)
-                    return (float)(y[q * YW + j + k] - y[q * YW + j]) +
-                           ((float)x[q * XW + j + k] - (float)x[q * XW + j]);
-                else
-                    return (float)((double)x[q * XW + j + k] - (double)x[q * XW + j]);
-            };
-            // upwind WENO7 face of component q about cell j of row x / y,
-            // stencil direction dir
-            auto face_r = [&](const TIN *x, const double *y, int q, int j, int dir) -> double {
-                if constexpr (INC) {
-                    const float corr =
-                        weno7_corr(dif(x, y, q, j, -3 * dir), dif(x, y, q, j, -2 * dir),
-                                   dif(x, y, q, j, -dir), dif(x, y, q, j, dir),
-                                   dif(x, y, q, j, 2 * dir), dif(x, y, q, j, 3 * dir));
-                    if constexpr (STAGE >= 2)  // Y + (D + correction)
-                        return y[q * YW + j] + (double)((float)x[q * XW + j] + corr);
-                    else
-                        return (double)x[q * XW + j] + (double)corr;
-                } else {
-                    return weno7_face(in_r(x, y, q, j - 3 * dir), in_r(x, y, q, j - 2 * dir),
-                                      in_r(x, y, q, j - dir), in_r(x, y, q, j),
-                                      in_r(x, y, q, j + dir), in_r(x, y, q, j + 2 * dir),
-                                      in_r(x, y, q, j + 3 * dir));
-                }
-            };
-            // FP64: numerator and denominator of that face (face = centre +
-            // num / den); the faces of components 0-3 and 4-7 of a row then
-            // share one division (recip4)
-            auto parts_r = [&](const TIN *x, const double *y, int q, int j, int dir, double &num,
-                               double &den) {
-                weno7_parts(in_r(x, y, q, j - 3 * dir), in_r(x, y, q, j - 2 * dir),
-                            in_r(x, y, q, j - dir), in_r(x, y, q, j), in_r(x, y, q, j + dir),
-                            in_r(x, y, q, j + 2 * dir), in_r(x, y, q, j + 3 * dir), num, den);
-            };
-
-            if constexpr (L::NE > 0) {
-                // edge faces of this chunk: warps 2ch, 2ch + 1 (mod R) in turn,
-                // lane -> (row 4h + lane / 8, component lane % 8).  Every lane
-                // arrives, also without advection, so the barrier's phases
-                // follow the ring.
-                const int h = (warp - L::NE * ch) & (R - 1);
-                if (h < L::NE) {
-                    const int r = h * (32 / NCOMP) + (lane >> 3), q = lane & (NCOMP - 1);
-                    if (advec) {
-                        const double v2 = __ldg(&a.vz[min(ch * R + r, a.nvz - 1)]);
-                        const int d2 = (v2 >= 0.0) ? 1 : -1;
-                        const int je = d2 > 0 ? -1 : TZ;
-                        if constexpr (INC) {
-                            s_edge[b][r][q] = face_r(xrow_of(r), yrow_of(r), q, je, d2);
-                        } else {
-                            // the row's four denominators of this component group
-                            // sit in lanes 4k..4k+3: the same division as the
-                            // neighbouring tile's own face, bit for bit
-                            double num, den, i[4];
-                            parts_r(xrow_of(r), yrow_of(r), q, je, d2, num, den);
-                            recip4(__shfl_sync(0xffffffffu, den, 0, 4),
-                                   __shfl_sync(0xffffffffu, den, 1, 4),
-                                   __shfl_sync(0xffffffffu, den, 2, 4),
-                                   __shfl_sync(0xffffffffu, den, 3, 4), i[0], i[1], i[2], i[3]);
-                            const int k = q & 3;
-                            const double inv = k == 0 ? i[0] : k == 1 ? i[1] : k == 2 ? i[2] : i[3];
-                            s_edge[b][r][q] = __fma_rn(num, inv, in_r(xrow_of(r), yrow_of(r), q, je));
-                        }
-                    }
-                    tma::mbar_arrive(&ebar[b]);
-                }
-            }
 
             double c[NCOMP], o[NCOMP], ko[NCOMP];
 #pragma unroll
             for (int q = 0; q < NCOMP; ++q) c[q] = in(q, lane);
-            if (SCHEME == FV) {
-                // upwind flux difference (rhs_fv.hpp:143-162): this lane's face
-                // and its neighbour's; the face at the tile's upwind edge comes
-                // from the chunk's edge warps (o[] holds the own faces meanwhile)
-                const int dir = (vzv >= 0.0) ? 1 : -1;
-                const int src = min(max(lane - dir, 0), TZ - 1);
-                if constexpr (INC) {
+            // FD: vacuum, matter, advection, (collective below), dissipation
 #pragma unroll
-                    for (int q = 0; q < NCOMP; ++q)
-                        o[q] = advec ? face_r(xrow, yrow, q, lane, dir) : 0.0;
-                } else {
-                    double den[NCOMP];
+            for (int q = 0; q < NCOMP; ++q) o[q] = 0.0;
+            if (a.flags & F_VAC) {
+                // read where used: batched, a is in shared memory and a
+                // per-tile copy would hold registers across the chunk loop
+                const double pmo = a.pmo, ct = a.ct, st = a.st;
+                o[EE] = -pmo * 2.0 * st * c[EXI];
+                o[XX] = pmo * 2.0 * st * c[EXI];
+                o[EXR] = -pmo * 2.0 * ct * c[EXI];
+                o[EXI] = pmo * (2.0 * ct * c[EXR] + st * (c[EE] - c[XX]));
+                o[BEE] = -pmo * 2.0 * st * c[BEXI];
+                o[BXX] = pmo * 2.0 * st * c[BEXI];
+                o[BEXR] = -pmo * 2.0 * ct * c[BEXI];
+                o[BEXI] = pmo * (2.0 * ct * c[BEXR] + st * (c[BEE] - c[BXX]));
+            }
+            if (a.flags & F_MAT) {
+                const double hm = a.Hm[z];
+                o[EXR] += hm * c[EXI];
+                o[EXI] += -hm * c[EXR];
+                o[BEXR] += -hm * c[BEXI];
+                o[BEXI] += hm * c[BEXR];
+            }
+            const int sv = (vzv > 0.0) - (vzv < 0.0);
+            const double ko_eps = a.ko_eps;
+            // one pass over each stencil: advection now, dissipation kept
+            // for after the collective term (the reference's order)
 #pragma unroll
-                    for (int q = 0; q < NCOMP; ++q) {
-                        o[q] = 0.0;
-                        den[q] = 1.0;
-                        if (advec) parts_r(xrow, yrow, q, lane, dir, o[q], den[q]);
+            for (int q = 0; q < NCOMP; ++q) {
+                const double m2 = in(q, lane - 2), m1 = in(q, lane - 1), p1 = in(q, lane + 1),
+                             p2 = in(q, lane + 2);
+                if (advec) {
+                    double adv;
+                    if (!GEN || a.fd_advec == 0) {
+                        adv = factor * ((m2 - p2) - 8.0 * (m1 - p1));
+                    } else if (a.fd_advec == 1) {
+                        adv = factor * (-4.0 * in(q, lane - 3 * sv) + 18.0 * in(q, lane - 2 * sv) -
+                                        36.0 * in(q, lane - sv) + 22.0 * c[q]);
+                    } else {
+                        adv = factor * (in(q, lane - 3 * sv) - 6.0 * in(q, lane - 2 * sv) +
+                                        18.0 * in(q, lane - sv) - 10.0 * c[q] -
+                                        3.0 * in(q, lane + sv));
                     }
-#pragma unroll
-                    for (int g = 0; g < NCOMP; g += 4) {
-                        double i[4];
-                        recip4(den[g], den[g + 1], den[g + 2], den[g + 3], i[0], i[1], i[2], i[3]);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            o[g + k] = advec ? __fma_rn(o[g + k], i[k], c[g + k]) : 0.0;
-                    }
+                    o[q] += adv;
                 }
-                if (advec) tma::mbar_wait(&ebar[b], (it / NBUF) & 1, err, 2, a0.wait_ns);
-#pragma unroll
-                for (int q = 0; q < NCOMP; ++q) {
-                    double adv = 0.0;
-                    if (advec) {
-                        const double fown = o[q];
-                        double fnb = __shfl_sync(0xffffffffu, fown, src);
-                        if ((dir > 0 && lane == 0) || (dir < 0 && lane == TZ - 1))
-                            fnb = s_edge[b][warp][q];
-                        if (open_bc) {
-                            // flux ghosts under OPEN_BC (updateBufferZone on rflux/lflux,
-                            // rhs_fv.hpp:118-119): rflux[-1] = rflux[0],
-                            // lflux[nz] = 2 lflux[nz-1] - lflux[nz-2]
-                            const double fm1 =
-                                __shfl_sync(0xffffffffu, fown, lane > 0 ? lane - 1 : 0);
-                            if (dir > 0 && z == 0) fnb = fown;
-                            if (dir < 0 && z == a.nz - 1) fnb = fown * 2.0 - fm1;
-                        }
-                        adv = dir > 0 ? factor * (fown - fnb) : factor * (fnb - fown);
-                    }
-                    o[q] = adv;
-                }
-                if (a.flags & F_VAC) {
-                    // read where used: batched, a is in shared memory and a
-                    // per-tile copy would hold registers across the chunk loop
-                    const double pmo = a.pmo, ct = a.ct, st = a.st;
-                    o[EE] += -2.0 * st * c[EXI] * pmo;
-                    o[XX] += 2.0 * st * c[EXI] * pmo;
-                    o[EXR] += -2.0 * ct * c[EXI] * pmo;
-                    o[EXI] += (2.0 * ct * c[EXR] + st * (c[EE] - c[XX])) * pmo;
-                    o[BEE] += -2.0 * st * c[BEXI] * pmo;
-                    o[BXX] += 2.0 * st * c[BEXI] * pmo;
-                    o[BEXR] += -2.0 * ct * c[BEXI] * pmo;
-                    o[BEXI] += (2.0 * ct * c[BEXR] + st * (c[BEE] - c[BXX])) * pmo;
-                }
-                if (a.flags & F_MAT) {
-                    const double hm = a.Hm[z];
-                    o[EXR] += hm * c[EXI];
-                    o[EXI] += -hm * c[EXR];
-                    o[BEXR] += -hm * c[BEXI];
-                    o[BEXI] += hm * c[BEXR];
-                }
-            } else {
-                // FD: vacuum, matter, advection, (collective below), dissipation
-#pragma unroll
-                for (int q = 0; q < NCOMP; ++q) o[q] = 0.0;
-                if (a.flags & F_VAC) {
-                    // read where used: batched, a is in shared memory and a
-                    // per-tile copy would hold registers across the chunk loop
-                    const double pmo = a.pmo, ct = a.ct, st = a.st;
-                    o[EE] = -pmo * 2.0 * st * c[EXI];
-                    o[XX] = pmo * 2.0 * st * c[EXI];
-                    o[EXR] = -pmo * 2.0 * ct * c[EXI];
-                    o[EXI] = pmo * (2.0 * ct * c[EXR] + st * (c[EE] - c[XX]));
-                    o[BEE] = -pmo * 2.0 * st * c[BEXI];
-                    o[BXX] = pmo * 2.0 * st * c[BEXI];
-                    o[BEXR] = -pmo * 2.0 * ct * c[BEXI];
-                    o[BEXI] = pmo * (2.0 * ct * c[BEXR] + st * (c[BEE] - c[BXX]));
-                }
-                if (a.flags & F_MAT) {
-                    const double hm = a.Hm[z];
-                    o[EXR] += hm * c[EXI];
-                    o[EXI] += -hm * c[EXR];
-                    o[BEXR] += -hm * c[BEXI];
-                    o[BEXI] += hm * c[BEXR];
-                }
-                const int sv = (vzv > 0.0) - (vzv < 0.0);
-                const double ko_eps = a.ko_eps;
-                // one pass over each stencil: advection now, dissipation kept
-                // for after the collective term (the reference's order)
-#pragma unroll
-                for (int q = 0; q < NCOMP; ++q) {
-                    const double m2 = in(q, lane - 2), m1 = in(q, lane - 1), p1 = in(q, lane + 1),
-                                 p2 = in(q, lane + 2);
-                    if (advec) {
-                        double adv;
-                        if (!GEN || a.fd_advec == 0) {
-                            adv = factor * ((m2 - p2) - 8.0 * (m1 - p1));
-                        } else if (a.fd_advec == 1) {
-                            adv = factor * (-4.0 * in(q, lane - 3 * sv) + 18.0 * in(q, lane - 2 * sv) -
-                                            36.0 * in(q, lane - sv) + 22.0 * c[q]);
-                        } else {
-                            adv = factor * (in(q, lane - 3 * sv) - 6.0 * in(q, lane - 2 * sv) +
-                                            18.0 * in(q, lane - sv) - 10.0 * c[q] -
-                                            3.0 * in(q, lane + sv));
-                        }
-                        o[q] += adv;
-                    }
-                    if (GEN && a.ko_order == 5)
-                        ko[q] = ko_eps * (in(q, lane - 3) + in(q, lane + 3) - 6.0 * (m2 + p2) +
-                                          15.0 * (m1 + p1) - 20.0 * c[q]);
-                    else
-                        ko[q] = ko_eps * (m2 + p2 - 4.0 * (m1 + p1) + 6.0 * c[q]);
-                }
+                if (GEN && a.ko_order == 5)
+                    ko[q] = ko_eps * (in(q, lane - 3) + in(q, lane + 3) - 6.0 * (m2 + p2) +
+                                      15.0 * (m1 + p1) - 20.0 * c[q]);
+                else
+                    ko[q] = ko_eps * (m2 + p2 - 4.0 * (m1 + p1) + 6.0 * c[q]);
             }
             if (coll) {
                 // this tile's input moments, read where used (they stay in
@@ -753,10 +341,8 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
                 o[BEXR] += mudv * ((c[BXX] - c[BEE]) * SA - c[BEXI] * SC);
                 o[BEXI] += mudv * ((c[BXX] - c[BEE]) * SB + c[BEXR] * SC);
             }
-            if (SCHEME == FD) {
 #pragma unroll
-                for (int q = 0; q < NCOMP; ++q) o[q] += ko[q];
-            }
+            for (int q = 0; q < NCOMP; ++q) o[q] += ko[q];
 
             // stage combine.  FP64 (stage values, A written once by stage 3 from
             // U in the A slot, U' and Y) or FP32-bulk (increments, common.cuh).
@@ -807,20 +393,9 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
                 }
             }
             // this warp is done with the buffer (after a failed wait it keeps
-            // the buffer: the producer's wait on it fails and it stops issuing;
-            // without a producer, the count never completes and no warp
-            // refills the buffer)
+            // the buffer: the producer's wait on it fails and it stops issuing)
             __syncwarp();
-            if (lane == 0 && landed) {
-                if constexpr (PW) {
-                    tma::mbar_arrive(&empty[b]);
-                } else if (ring_release_count(&s_cnt[b]) == (it / NBUF) * R + (R - 1)) {
-                    // the last of the R warps to release buffer b: its next chunk
-                    fence_proxy_async_smem();
-                    int t2 = t, ch2 = ch;
-                    if (advance(t2, ch2, NBUF)) issue_at(t2, ch2, it + NBUF);
-                }
-            }
+            if (lane == 0 && landed) tma::mbar_arrive(&empty[b]);
 
             TOUT uleft[NCOMP];
             if (open_bc) {
@@ -857,38 +432,18 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
                     const double Am = um[EXI] + um[BEXI];
                     const double Bm = um[EXR] - um[BEXR];
                     const double Cm = um[EE] - um[XX] - um[BEE] + um[BXX];
-                    if constexpr (L::MSM) {
-                        s_red[warp][0][lane] += Am;
-                        s_red[warp][1][lane] += Bm;
-                        s_red[warp][2][lane] += Cm;
-                        s_red[warp][3][lane] += vzv * Am;
-                        s_red[warp][4][lane] += vzv * Bm;
-                        s_red[warp][5][lane] += vzv * Cm;
-                    } else {
-                        macc[0] += Am;
-                        macc[1] += Bm;
-                        macc[2] += Cm;
-                        macc[3] += vzv * Am;
-                        macc[4] += vzv * Bm;
-                        macc[5] += vzv * Cm;
-                    }
+                    macc[0] += Am;
+                    macc[1] += Bm;
+                    macc[2] += Cm;
+                    macc[3] += vzv * Am;
+                    macc[4] += vzv * Bm;
+                    macc[5] += vzv * Cm;
                 }
             }
         }
         // tile epilogue: output moments (fixed-order sum over warps) and the
         // next tile's input moments
-        if ((coll || BATCHED) && L::MSM) {
-            consumer_sync();
-            if (tid < NMOM * TZ) {
-                const int m = tid / TZ, zz = tid % TZ;
-                double s = 0.0;
-#pragma unroll
-                for (int w = 0; w < R; ++w) s += s_red[w][m][zz];
-                if (coll) a.Mout[(long long)m * a.nz + z0 + zz] = s;
-                s_mom[m][zz] = mnext;  // every consumer read this tile's values above
-            }
-            consumer_sync();
-        } else if (coll || BATCHED) {
+        if (coll || BATCHED) {
             // warps w and w + R/2 pair up, then the R/2 pair sums are added
             // in a fixed order
             if (warp >= R / 2) {
@@ -912,15 +467,6 @@ __global__ void __launch_bounds__(tma::producer_warp<SCHEME, BATCHED>()
             consumer_sync();
         }
         cur = nxt;
-    }
-    if constexpr (!PW) {
-        // the last copies issued into each buffer have landed before the block
-        // exits (in normal operation the consumers have waited for them)
-        consumer_sync();
-        if (tid == 0)
-            for (int b = 0; b < NBUF; ++b)
-                if (s_last[b] >= 0)
-                    tma::mbar_drain(&full[b], ((uint32_t)s_last[b] / NBUF) & 1, err, a0.wait_ns);
     }
 }
 
@@ -965,44 +511,35 @@ int make_state_map(CUtensorMap *map, const void *base, int elem_bytes, int ld, i
     return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
-int tma_box_x(int elem_bytes) { return elem_bytes == 8 ? tma::xw<double>() : tma::xw<float>(); }
+// Width of the input box of a halo operand; FP64 stage 3 of FD (`narrow`)
+// reads its stage input in 40-cell rows (Layout).
+int tma_box_x(int scheme, int elem_bytes, bool narrow)
+{
+    if (scheme == FV) return fv_box_x(elem_bytes);
+    if (narrow) return tma::TZ + 2 * tma::HALO;
+    return elem_bytes == 8 ? tma::xw<double>() : tma::xw<float>();
+}
 int tma_box_tile() { return tma::TZ; }
 // Rows of a map's box: `wide` for the operands of the 12-row FD stages.
 int tma_box_rows(int scheme, bool wide) { return scheme == FD && wide ? 12 : 8; }
 // largest nvz the TMA layout is offered for (the range its tests cover; the
-// kernel itself keeps no per-row state in shared memory)
+// kernels themselves keep no per-row state in shared memory)
 int tma_max_nvz() { return TMA_MAX_NVZ; }
 
-static const int TMA_SMEM_MAX = 232448;  // opt-in shared memory per block on sm_100
-static const int TMA_SMEM_SM = 233472;   // shared memory per SM (1 KB reserved per block)
-
 // Shared memory of one block with an NB-deep ring.
-template <int SCHEME, class TIN, class TOUT, int STAGE>
+template <class TIN, class TOUT, int STAGE>
 static int tma_smem(int NB)
 {
-    using L = tma::Layout<SCHEME, TIN, TOUT, STAGE>;
-    return NB * L::BUF + (2 + (L::NE ? 1 : 0)) * NB * 8 + (1 + L::NRED) * NMOM * tma::TZ * 8 +
-           (L::NE ? NB * L::R * NCOMP * 8 : 0) +
-           (int)sizeof(StageArgs) + NB * 8;  // + release counts, last chunks
+    using L = tma::Layout<TIN, TOUT, STAGE>;
+    return NB * L::BUF + 2 * NB * 8 + (1 + L::NRED) * NMOM * tma::TZ * 8 + (int)sizeof(StageArgs);
 }
 
-static int tma_smem_limit(int minb)
-{
-    return minb == 1 ? TMA_SMEM_MAX : TMA_SMEM_SM / minb - 1024;
-}
-
-// The operand maps of one launch: X (stage input with halo), Y, A and B (see
-// Layout; unused ones are ignored).
-struct StageMaps {
-    const CUtensorMap *x, *y, *a, *b;
-};
-
-template <int SCHEME, bool GEN, int STAGE, class TIN, class TOUT, int NB, int MINB>
-static cudaError_t launch_nb(const StageMaps &m, const StageArgs &a, int *err, int nblocks,
+template <bool GEN, int STAGE, class TIN, class TOUT, int NB, int MINB>
+static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *err, int nblocks,
                              cudaStream_t s, const BatchDev *bd)
 {
-    auto kern = rk4_stage_tma_kernel<SCHEME, GEN, STAGE, TIN, TOUT, NB, false, MINB>;
-    auto kernb = rk4_stage_tma_kernel<SCHEME, GEN, STAGE, TIN, TOUT, NB, true, MINB>;
+    auto kern = rk4_stage_tma_kernel<GEN, STAGE, TIN, TOUT, NB, false, MINB>;
+    auto kernb = rk4_stage_tma_kernel<GEN, STAGE, TIN, TOUT, NB, true, MINB>;
     if (nblocks <= 0) {  // preparation call: shared-memory limit and carveout
         for (auto k : {kern, kernb}) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1014,9 +551,8 @@ static cudaError_t launch_nb(const StageMaps &m, const StageArgs &a, int *err, i
         }
         return cudaSuccess;
     }
-    const int shmem = tma_smem<SCHEME, TIN, TOUT, STAGE>(NB);
-    using L = tma::Layout<SCHEME, TIN, TOUT, STAGE>;
-    constexpr int NT = tma::producer_warp<SCHEME, false>() ? L::NTHR : L::NTHR_NP;
+    const int shmem = tma_smem<TIN, TOUT, STAGE>(NB);
+    constexpr int NT = tma::Layout<TIN, TOUT, STAGE>::NTHR;
     if (bd)
         kernb<<<nblocks, NT, shmem, s>>>(*m.x, *m.y, *m.a, *m.b, a, err, *bd);
     else
@@ -1044,31 +580,18 @@ static int tma_ring_env()
 template <class TIN, class TOUT, int STAGE>
 static int tma_fd_ring()
 {
-    using L = tma::Layout<FD, TIN, TOUT, STAGE>;
+    using L = tma::Layout<TIN, TOUT, STAGE>;
     int nb = 2;
     while (nb < 4 && (nb + 1) * L::BUF <= 144 * 1024) ++nb;
     const int e = tma_ring_env();
     if (e) nb = e;
-    while (nb > 2 && tma_smem<FD, TIN, TOUT, STAGE>(nb) > tma_smem_limit(1)) --nb;
+    while (nb > 2 && tma_smem<TIN, TOUT, STAGE>(nb) > tma_smem_limit(1)) --nb;
     return nb;
 }
 
-// Blocks per SM.  FD (memory bound): one, with the deepest ring that fits.
-// FV (FP64 bound, 8 warps per block): two, to hide FP64 and shared-memory
-// latency with twice the warps, each with the deepest ring that fits in half
-// the SM (COSENU_TMA_MINB=1 selects one block per SM with a 4-deep ring).
-static int tma_minb_env()
-{
-    static int v = -1;
-    if (v < 0) {
-        const char *e = getenv("COSENU_TMA_MINB");
-        v = (e && e[0] == '1') ? 1 : 2;
-    }
-    return v;
-}
-
-// FD: COSENU_TMA_MINB_FD=2 runs two blocks per SM (<= 112 registers each,
-// half the shared memory) instead of one.
+// Blocks per SM.  FD (memory bound): one, with the deepest ring that fits;
+// COSENU_TMA_MINB_FD=2 runs two blocks per SM (<= 112 registers each, half the
+// shared memory) instead.
 static int tma_minb_fd_env()
 {
     static int v = -1;
@@ -1079,72 +602,66 @@ static int tma_minb_fd_env()
     return v;
 }
 
-int tma_blocks_per_sm(int scheme) { return scheme == FV ? tma_minb_env() : tma_minb_fd_env(); }
+int tma_blocks_per_sm(int scheme) { return scheme == FV ? fv_blocks_per_sm() : tma_minb_fd_env(); }
 
-template <int SCHEME, bool GEN, int STAGE, class TIN, class TOUT>
-static cudaError_t launch_one(const StageMaps &m, const StageArgs &a, int *err, int nblocks,
+template <bool GEN, int STAGE, class TIN, class TOUT>
+static cudaError_t launch_one(const tma::StageMaps &m, const StageArgs &a, int *err, int nblocks,
                               cudaStream_t s, const BatchDev *bd)
 {
-#define LNB(NB, MINB) launch_nb<SCHEME, GEN, STAGE, TIN, TOUT, NB, MINB>(m, a, err, nblocks, s, bd)
-    if constexpr (SCHEME == FD) {
-        if (nblocks <= 0) {
-            cudaError_t e = LNB(2, 1);
-            if (e == cudaSuccess) e = LNB(3, 1);
-            if (e == cudaSuccess) e = LNB(4, 1);
-            if (e == cudaSuccess) e = LNB(2, 2);
-            if (e == cudaSuccess) e = LNB(3, 2);
-            if (e == cudaSuccess) e = LNB(4, 2);
-            return e;
-        }
-        if (tma_minb_fd_env() == 2) {
-            const int lim = tma_smem_limit(2);
-            if (tma_smem<SCHEME, TIN, TOUT, STAGE>(4) <= lim) return LNB(4, 2);
-            if (tma_smem<SCHEME, TIN, TOUT, STAGE>(3) <= lim) return LNB(3, 2);
-            return LNB(2, 2);
-        }
-        switch (tma_fd_ring<TIN, TOUT, STAGE>()) {
-        case 2: return LNB(2, 1);
-        case 3: return LNB(3, 1);
-        default: return LNB(4, 1);
-        }
-    } else {
-        if (nblocks <= 0) {
-            cudaError_t e = LNB(4, 1);
-            if (e == cudaSuccess) e = LNB(4, 2);
-            if (e == cudaSuccess) e = LNB(3, 2);
-            if (e == cudaSuccess) e = LNB(2, 2);
-            return e;
-        }
-        if (tma_minb_env() == 1) return LNB(4, 1);
+#define LNB(NB, MINB) launch_nb<GEN, STAGE, TIN, TOUT, NB, MINB>(m, a, err, nblocks, s, bd)
+    if (nblocks <= 0) {
+        cudaError_t e = LNB(2, 1);
+        if (e == cudaSuccess) e = LNB(3, 1);
+        if (e == cudaSuccess) e = LNB(4, 1);
+        if (e == cudaSuccess) e = LNB(2, 2);
+        if (e == cudaSuccess) e = LNB(3, 2);
+        if (e == cudaSuccess) e = LNB(4, 2);
+        return e;
+    }
+    if (tma_minb_fd_env() == 2) {
         const int lim = tma_smem_limit(2);
-        if (tma_smem<SCHEME, TIN, TOUT, STAGE>(4) <= lim) return LNB(4, 2);
-        if (tma_smem<SCHEME, TIN, TOUT, STAGE>(3) <= lim) return LNB(3, 2);
+        if (tma_smem<TIN, TOUT, STAGE>(4) <= lim) return LNB(4, 2);
+        if (tma_smem<TIN, TOUT, STAGE>(3) <= lim) return LNB(3, 2);
         return LNB(2, 2);
+    }
+    switch (tma_fd_ring<TIN, TOUT, STAGE>()) {
+    case 2: return LNB(2, 1);
+    case 3: return LNB(3, 1);
+    default: return LNB(4, 1);
     }
 #undef LNB
 }
 
-template <int SCHEME, bool GEN>
-static cudaError_t launch_p(const StageMaps &m, const StageArgs &a, int stage, int fp32, int *err,
-                            int nblocks, cudaStream_t s, const BatchDev *bd)
+template <bool GEN>
+static cudaError_t launch_p(const tma::StageMaps &m, const StageArgs &a, int stage, int fp32,
+                            int *err, int nblocks, cudaStream_t s, const BatchDev *bd)
 {
     if (fp32) {
         // FP32-bulk: Y in, D1 out; Y + D1 in, D2 out; Y + D2 in, D3 out; Y + D3 in, Y' out
         switch (stage) {
-        case 1: return launch_one<SCHEME, GEN, 1, double, float>(m, a, err, nblocks, s, bd);
-        case 2: return launch_one<SCHEME, GEN, 2, float, float>(m, a, err, nblocks, s, bd);
-        case 3: return launch_one<SCHEME, GEN, 3, float, float>(m, a, err, nblocks, s, bd);
-        case 4: return launch_one<SCHEME, GEN, 4, float, double>(m, a, err, nblocks, s, bd);
+        case 1: return launch_one<GEN, 1, double, float>(m, a, err, nblocks, s, bd);
+        case 2: return launch_one<GEN, 2, float, float>(m, a, err, nblocks, s, bd);
+        case 3: return launch_one<GEN, 3, float, float>(m, a, err, nblocks, s, bd);
+        case 4: return launch_one<GEN, 4, float, double>(m, a, err, nblocks, s, bd);
         }
     } else {
         switch (stage) {
-        case 1: return launch_one<SCHEME, GEN, 1, double, double>(m, a, err, nblocks, s, bd);
-        case 2: return launch_one<SCHEME, GEN, 2, double, double>(m, a, err, nblocks, s, bd);
-        case 3: return launch_one<SCHEME, GEN, 3, double, double>(m, a, err, nblocks, s, bd);
-        case 4: return launch_one<SCHEME, GEN, 4, double, double>(m, a, err, nblocks, s, bd);
+        case 1: return launch_one<GEN, 1, double, double>(m, a, err, nblocks, s, bd);
+        case 2: return launch_one<GEN, 2, double, double>(m, a, err, nblocks, s, bd);
+        case 3: return launch_one<GEN, 3, double, double>(m, a, err, nblocks, s, bd);
+        case 4: return launch_one<GEN, 4, double, double>(m, a, err, nblocks, s, bd);
         }
     }
     return cudaErrorInvalidValue;
+}
+
+static cudaError_t launch_any(const tma::StageMaps &m, const StageArgs &a, int scheme, int stage,
+                              int fp32, int *err, int nblocks, cudaStream_t s, const BatchDev *bd)
+{
+    if (scheme == FV) return launch_fv_tma(m, a, stage, fp32, err, nblocks, s, bd);
+    const bool gen = a.fd_advec != 0 || a.ko_order == 5;
+    return gen ? launch_p<true>(m, a, stage, fp32, err, nblocks, s, bd)
+               : launch_p<false>(m, a, stage, fp32, err, nblocks, s, bd);
 }
 
 cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
@@ -1152,11 +669,8 @@ cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
                                  int scheme, int stage, int fp32, int *err, int nblocks,
                                  cudaStream_t s)
 {
-    const StageMaps m{&mX, &mY, &mA, &mB};
-    if (scheme == FV) return launch_p<FV, false>(m, a, stage, fp32, err, nblocks, s, nullptr);
-    const bool gen = a.fd_advec != 0 || a.ko_order == 5;
-    return gen ? launch_p<FD, true>(m, a, stage, fp32, err, nblocks, s, nullptr)
-               : launch_p<FD, false>(m, a, stage, fp32, err, nblocks, s, nullptr);
+    const tma::StageMaps m{&mX, &mY, &mA, &mB};
+    return launch_any(m, a, scheme, stage, fp32, err, nblocks, s, nullptr);
 }
 
 // Ensemble launch: `a` carries the variant switches shared by every instance
@@ -1166,11 +680,8 @@ cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, i
                                        cudaStream_t s)
 {
     CUtensorMap z{};
-    const StageMaps m{&z, &z, &z, &z};
-    if (scheme == FV) return launch_p<FV, false>(m, a, stage, fp32, err, nblocks, s, &bd);
-    const bool gen = a.fd_advec != 0 || a.ko_order == 5;
-    return gen ? launch_p<FD, true>(m, a, stage, fp32, err, nblocks, s, &bd)
-               : launch_p<FD, false>(m, a, stage, fp32, err, nblocks, s, &bd);
+    const tma::StageMaps m{&z, &z, &z, &z};
+    return launch_any(m, a, scheme, stage, fp32, err, nblocks, s, &bd);
 }
 
 // Sets the shared-memory attribute of every instantiation on the current device.

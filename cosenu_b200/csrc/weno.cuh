@@ -5,102 +5,131 @@
 
 namespace cosenu {
 
-// WENO7 face value from the 7-point stencil a..g = u[-3..3] about the cell
-// whose right face (j+1/2) is reconstructed with left-biased weights
-// (rflux of src/rhs_fv.hpp:37-71).  Smoothness indicators and candidate
-// polynomials of the four 4-point sub-stencils; nonlinear weights
-// gamma_r / (eps + beta_r)^2 with gamma = (4, 18, 12, 1)/35 and eps = 1e-6.
-// FP64: the indicators and the candidate values are evaluated on differences
-// from the centre value d (the indicators are invariant under a constant
-// shift and each candidate's weights sum to 12, so the face is d plus the
-// weighted differences: 15 fewer FP64 operations per face and less
-// cancellation), and the four weights are brought to a common denominator,
-// so that the face is d + num / den.  gamma and the 12 ride on the
-// candidates' coefficients (gamma_r / 12 x the integer weights) and gamma on
-// den, not on the weights; den = 4 w0 + 18 w1 + 12 w2 + w3 is three FMAs.
-__device__ __forceinline__ void weno7_parts(double a, double b, double c, double d, double e,
-                                            double f, double g, double &num, double &den)
+// The face value of the cell whose right face (j+1/2) is reconstructed with
+// left-biased weights (rflux of src/rhs_fv.hpp:37-71), from the six first
+// differences dl[i] = u[i-2] - u[i-3] (i = 0..5) of its seven-point stencil
+// u[-3..3]: smoothness indicators and candidate polynomials of the four
+// 4-point sub-stencils, nonlinear weights gamma_r / (eps + beta_r)^2 with
+// gamma = (4, 18, 12, 1)/35 and eps = 1e-6.  The mirrored stencil (the left
+// face of a cell with downwind weights) has the same differences in reverse
+// order with the opposite sign; every term below is then even (the
+// indicators) or odd (the correction), so the caller passes them reversed and
+// subtracts the correction.
+//
+// FP64 issue bounds the FV stages, so the indicators are written as the sums of
+// squares they are, not as quadratic forms in the values: with the second,
+// third and fourth differences D, T, F,
+//     beta_r / 60 = y_r^2 + 13/3 D_r^2 + 781/180 T_r^2,
+// where y_r and D_r are twice the first and second derivative of sub-stencil
+// r's cubic at the centre (the constant 60 cancels in the weights), and
+// neighbouring candidates differ by one fourth difference:
+//     q0 = q1 + Fa,  q2 = q1 + Fb,  q3 = q2 - 3 Fc.
+// 70 FP64 operations for a lone face, but D, T, F and the T^2 terms are those
+// of the neighbouring faces too: 55 per face for four consecutive faces of one
+// row evaluated by one thread (the compiler merges the equal expressions),
+// against 75 in the quadratic form, which shares nothing.
+constexpr double WENO_EPS = 1e-6 / 60.0;
+
+template <class T> struct WenoB {
+    T b0, b1, b2, b3;  // eps + beta_r, over 60
+    T Fa, Fb, Fc;      // fourth differences about centre + 1, centre, centre - 1
+    T q1;              // 12 x (candidate 1 - centre value)
+};
+
+template <class T> __device__ __forceinline__ WenoB<T> weno7_indicators(const T *dl)
 {
-    const double eps = 1e-6;
-    const double A = a - d, B = b - d, Cc = c - d, E = e - d, F = f - d, G = g - d;
-    double s0 = E * (11003. * E - 17246. * F + 4642. * G) + F * (7043. * F - 3882. * G) +
-                547. * G * G;
-    double s1 = Cc * (547. * Cc + 1922. * E - 494. * F) + E * (2843. * E - 1642. * F) +
-                267. * F * F;
-    double s2 = B * (267. * B - 1642. * Cc - 494. * E) + Cc * (2843. * Cc + 1922. * E) +
-                547. * E * E;
-    double s3 = A * (547. * A - 3882. * B + 4642. * Cc) + B * (7043. * B - 17246. * Cc) +
-                11003. * Cc * Cc;
-    // gamma_r x (candidate value - d): 12 x (candidate - d) has integer
-    // weights summing to 12, scaled here by gamma_r / 12 = 1/3, 3/2, 1, 1/12
-    double q0 = (13. / 3.) * E - (5. / 3.) * F + (1. / 3.) * G;
-    double q1 = -1.5 * Cc + 10.5 * E - 1.5 * F;
-    double q2 = B - 5. * Cc + 3. * E;
-    double q3 = -0.25 * A + (13. / 12.) * B - (23. / 12.) * Cc;
-    double d0 = (eps + s0) * (eps + s0);
-    double d1 = (eps + s1) * (eps + s1);
-    double d2 = (eps + s2) * (eps + s2);
-    double d3 = (eps + s3) * (eps + s3);
-    double d01 = d0 * d1, d23 = d2 * d3;
-    // the weights without gamma: w_r = prod_{k != r} d_k
-    double w0 = d1 * d23, w1 = d0 * d23, w2 = d01 * d3, w3 = d01 * d2;
-    num = w0 * q0 + w1 * q1 + w2 * q2 + w3 * q3;
-    den = w3 + 4. * w0 + 18. * w1 + 12. * w2;
+    const T c13 = T(13.0 / 3.0), c781 = T(781.0 / 180.0), eps = T(WENO_EPS);
+    const T D0 = dl[1] - dl[0], D1 = dl[2] - dl[1], D2 = dl[3] - dl[2], D3 = dl[4] - dl[3],
+            D4 = dl[5] - dl[4];
+    const T T0 = D1 - D0, T1 = D2 - D1, T2 = D3 - D2, T3 = D4 - D3;
+    const T t0 = (c781 * T0) * T0 + eps, t1 = (c781 * T1) * T1 + eps, t2 = (c781 * T2) * T2 + eps,
+            t3 = (c781 * T3) * T3 + eps;
+    const T C2 = dl[2] + dl[3];       // u[1] - u[-1]
+    const T dd = (c13 * D2) * D2;     // the inner sub-stencils' second difference
+    const T y1 = C2 - T(1.0 / 3.0) * T2, y2 = C2 - T(1.0 / 3.0) * T1;
+    const T e0 = D3 - T3, e3 = D1 + T0;  // the outer ones', continued to the centre
+    const T y0 = (T(2) * dl[3] - D3) + T(2.0 / 3.0) * T3;
+    const T y3 = (T(2) * dl[2] + D1) + T(2.0 / 3.0) * T0;
+    WenoB<T> r;
+    r.b0 = (c13 * e0) * e0 + (y0 * y0 + t3);
+    r.b1 = (y1 * y1 + dd) + t2;
+    r.b2 = (y2 * y2 + dd) + t1;
+    r.b3 = (c13 * e3) * e3 + (y3 * y3 + t0);
+    r.Fc = T1 - T0;
+    r.Fb = T2 - T1;
+    r.Fa = T3 - T2;
+    r.q1 = T(6) * dl[3] + (dl[2] - dl[4]);
+    return r;
 }
 
-__device__ __forceinline__ double weno7_face(double a, double b, double c, double d, double e,
-                                             double f, double g)
+// FP64: the weights brought to a common denominator; the face is
+// centre + (q1 + num / den) / 12.
+__device__ __forceinline__ void weno7_parts(const double *dl, double &q1, double &num, double &den)
 {
-    double num, den;
-    weno7_parts(a, b, c, d, e, f, g, num, den);
-    return d + num / den;
+    const WenoB<double> r = weno7_indicators<double>(dl);
+    const double d0 = r.b0 * r.b0, d1 = r.b1 * r.b1, d2 = r.b2 * r.b2, d3 = r.b3 * r.b3;
+    const double d01 = d0 * d1, d23 = d2 * d3;
+    // gamma_r x prod_{k != r} d_k
+    const double w0 = 4. * (d1 * d23), w1 = d0 * d23, w2 = 12. * (d01 * d3), w3 = d01 * d2;
+    q1 = r.q1;
+    num = w0 * r.Fa + w2 * r.Fb + w3 * (r.Fb - 3. * r.Fc);
+    den = (18. * w1 + w0) + (w2 + w3);
+}
+
+// 12 x (face - centre), one face.
+__device__ __forceinline__ double weno7_corr12(const double *dl)
+{
+    double q1, num, den;
+    weno7_parts(dl, q1, num, den);
+    return q1 + num / den;
 }
 
 // 1 / D0 .. 1 / D3 from one division: the product of the four, its
 // reciprocal, then products of the others.  Denominators of weno7_parts lie
-// in [3e-35, 2e33] where the stencil differences are at most 2 in magnitude
+// in [7e-46, 1e21] where the stencil differences are at most 2 in magnitude
 // (density-matrix entries of O(1)), so the product of four stays far inside
-// the FP64 range.  Explicit round-to-nearest operations: the same
-// inputs give the same bits wherever this is evaluated (the face of a tile's
-// edge row is computed by two different warps).
+// the FP64 range.
 __device__ __forceinline__ void recip4(double D0, double D1, double D2, double D3, double &i0,
                                        double &i1, double &i2, double &i3)
 {
-    const double p01 = __dmul_rn(D0, D1), p23 = __dmul_rn(D2, D3);
-    const double r = 1.0 / __dmul_rn(p01, p23);
-    const double r01 = __dmul_rn(r, p23), r23 = __dmul_rn(r, p01);
-    i0 = __dmul_rn(r01, D1);
-    i1 = __dmul_rn(r01, D0);
-    i2 = __dmul_rn(r23, D3);
-    i3 = __dmul_rn(r23, D2);
+    const double p01 = D0 * D1, p23 = D2 * D3;
+    const double r = 1.0 / (p01 * p23);
+    const double r01 = r * p23, r23 = r * p01;
+    i0 = r01 * D1;
+    i1 = r01 * D0;
+    i2 = r23 * D3;
+    i3 = r23 * D2;
 }
 
-// FP32-bulk form: the face value minus the centre value from the six
-// stencil differences A..G = u[-3..3] - u[0] (skipping the centre), which the
-// caller takes in FP64 so that FP32 sees only the small differences and not
-// the O(1) values.  Same indicators, candidates and weights as above; the
-// weights use fast reciprocals.
-__device__ __forceinline__ float weno7_corr(float A, float B, float Cc, float E, float F, float G)
+// 12 x (face - centre) of four consecutive faces from the nine differences of
+// their ten cells.
+__device__ __forceinline__ void weno7_quad(const double *dl, double *c12)
 {
-    const float eps = 1e-6f;
-    float s0 = E * (11003.f * E - 17246.f * F + 4642.f * G) + F * (7043.f * F - 3882.f * G) +
-               547.f * G * G;
-    float s1 = Cc * (547.f * Cc + 1922.f * E - 494.f * F) + E * (2843.f * E - 1642.f * F) +
-               267.f * F * F;
-    float s2 = B * (267.f * B - 1642.f * Cc - 494.f * E) + Cc * (2843.f * Cc + 1922.f * E) +
-               547.f * E * E;
-    float s3 = A * (547.f * A - 3882.f * B + 4642.f * Cc) + B * (7043.f * B - 17246.f * Cc) +
-               11003.f * Cc * Cc;
-    float q0 = 13.f * E - 5.f * F + G;
-    float q1 = -Cc + 7.f * E - F;
-    float q2 = B - 5.f * Cc + 3.f * E;
-    float q3 = -3.f * A + 13.f * B - 23.f * Cc;
-    float w0 = __fdividef(4.f, (eps + s0) * (eps + s0));
-    float w1 = __fdividef(18.f, (eps + s1) * (eps + s1));
-    float w2 = __fdividef(12.f, (eps + s2) * (eps + s2));
-    float w3 = __fdividef(1.f, (eps + s3) * (eps + s3));
-    float num = w0 * q0 + w1 * q1 + w2 * q2 + w3 * q3;
-    return __fdividef(num, 12.f * (w0 + w1 + w2 + w3));
+    double q1[4], num[4], den[4], inv[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) weno7_parts(dl + k, q1[k], num[k], den[k]);
+    recip4(den[0], den[1], den[2], den[3], inv[0], inv[1], inv[2], inv[3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c12[k] = num[k] * inv[k] + q1[k];
+}
+
+// FP32-bulk form: 12 x (face - centre) in FP32 from differences the caller
+// takes in FP64, so that FP32 sees only the small differences and not the
+// O(1) values.  Same indicators and candidates; the weights use fast
+// reciprocals (a common denominator would leave the FP32 range).
+__device__ __forceinline__ float weno7_corr12(const float *dl)
+{
+    const WenoB<float> r = weno7_indicators<float>(dl);
+    const float w0 = __fdividef(4.f, r.b0 * r.b0), w1 = __fdividef(18.f, r.b1 * r.b1),
+                w2 = __fdividef(12.f, r.b2 * r.b2), w3 = __fdividef(1.f, r.b3 * r.b3);
+    const float num = w0 * r.Fa + w2 * r.Fb + w3 * (r.Fb - 3.f * r.Fc);
+    return r.q1 + __fdividef(num, (w0 + w1) + (w2 + w3));
+}
+
+__device__ __forceinline__ void weno7_quad(const float *dl, float *c12)
+{
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c12[k] = weno7_corr12(dl + k);
 }
 
 }  // namespace cosenu
