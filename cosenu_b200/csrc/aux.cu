@@ -56,7 +56,8 @@ __global__ void __launch_bounds__(NTHREADS) moments_kernel(const double *__restr
     int z0 = blockIdx.x * TZ, z = z0 + lz, vt = blockIdx.y;
     int vbeg = vt * tv, vend = min(vbeg + tv, nvz);
     double acc[NMOM] = {0, 0, 0, 0, 0, 0};
-    for (int v = vbeg + rr; v < vend; v += RP) {
+    // (the last tile of a row may be partial)
+    for (int v = vbeg + rr; v < vend && z < nz; v += RP) {
         long long o = (long long)v * ld + HP + z;
         double A = X[EXI * cs + o] + X[BEXI * cs + o];
         double B = X[EXR * cs + o] - X[BEXR * cs + o];
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(NTHREADS) moments_kernel(const double *__restr
         int m = q / TZ, zz = q % TZ;
         double s = 0.0;
         for (int t = 0; t < RP; ++t) s += s_red[t][m][zz];
-        M[((long long)vt * NMOM + m) * nz + z0 + zz] = s;
+        if (z0 + zz < nz) M[((long long)vt * NMOM + m) * nz + z0 + zz] = s;
     }
 }
 
@@ -328,7 +329,7 @@ cudaError_t launch_ghost_fill(double *buf, long long cs, int ld, int nz, int nvz
 cudaError_t launch_moments(const double *X, double *M, const double *vz, long long cs, int ld,
                            int nz, int nvz, int tz, int tv, cudaStream_t s)
 {
-    dim3 grid(nz / tz, (nvz + tv - 1) / tv);
+    dim3 grid((nz + tz - 1) / tz, (nvz + tv - 1) / tv);
     switch (tz) {
     case 8: moments_kernel<8><<<grid, NTHREADS, 0, s>>>(X, M, vz, cs, ld, nz, nvz, tv); break;
     case 16: moments_kernel<16><<<grid, NTHREADS, 0, s>>>(X, M, vz, cs, ld, nz, nvz, tv); break;

@@ -11,8 +11,8 @@
 //
 // Step counts are known up front, so a run is a sequence of phases: each
 // phase advances the members that are still active by the smallest remaining
-// count, with the per-step launches captured once into a CUDA graph and
-// replayed; finished members drop out of the table between phases.
+// count (long phases as replays of a captured CUDA graph); finished members
+// drop out of the table between phases.
 //
 // FP32-bulk members write each step's new state into their other FP64 buffer
 // (common.cuh), so stage arguments and tensor maps exist per buffer parity.
@@ -54,6 +54,7 @@ struct cosenu_batch {
     int tz = 32;       // register-tiled z tile
     std::vector<int> tv;  // register-tiled v tile per member
     int max_nvz = 0;
+    int piece = 1;  // FV, TMA family: chunks of 8 rows per table entry at most
     std::vector<cudaGraphExec_t> graphs;  // executed graphs, released after a synchronize
     std::string err;
 };
@@ -91,24 +92,53 @@ int upload_args(cosenu_batch *b)
     return COSENU_OK;
 }
 
-// Table of tiles of the members in `active`.  TMA family: member by member
-// (a block then streams consecutive z tiles of one member), with `ranges`
-// splitting the table into nblk contiguous pieces of equal work; register-
-// tiled family: heaviest tiles first (one block per entry).
+// Pieces of an FV z tile: up to b->piece chunks of 8 rows each (the same cut in
+// every phase: a stage sums the moments that the previous launch wrote piece by
+// piece).
+int fv_pieces(const cosenu_batch *b, int i) { return ((b->m[i]->p.nvz + 7) / 8 + b->piece - 1) / b->piece; }
+
+// Table of the work of the members in `active`, member by member.  TMA family,
+// FD: one entry per z tile, `ranges` splitting the table into at most max_blk
+// contiguous runs of equal work.  TMA family, FV: one entry per piece of a z
+// tile, dealt out over the blocks along z within a v band, so that the blocks
+// running together read neighbouring cells (16 members of 512-4096 cells:
+// 0.592 ms a step against 0.616 in contiguous runs).  Register-tiled family:
+// heaviest tiles first (one block per entry).
 size_t build_table(cosenu_batch *b, const std::vector<int> &active, std::vector<int4> &out,
-                   std::vector<int> *ranges = nullptr, int nblk = 0)
+                   std::vector<int> *ranges = nullptr, int max_blk = 0)
 {
     out.clear();
     if (b->use_tma) {
         std::vector<long long> w;
         for (int i : active) {
             const cosenu_params &p = b->m[i]->p;
-            for (int zt = 0; zt < p.nz / 32; ++zt) {
-                out.push_back(make_int4(i, zt, 0, p.nvz));  // .w: rows, read by the kernel
-                w.push_back((long long)(p.nvz + 7) / 8 + 1);  // chunks + per-tile overhead
+            const int nch = (p.nvz + 7) / 8;
+            if (b->scheme == COSENU_FD) {
+                for (int zt = 0; zt < p.nz / 32; ++zt) {
+                    out.push_back(make_int4(i, zt, 0, p.nvz));  // .w: rows
+                    w.push_back(nch + 1);                       // chunks + per-tile overhead
+                }
+                continue;
+            }
+            const int np = fv_pieces(b, i);
+            for (int k = 0; k < np; ++k) {
+                const int c0 = k * b->piece, c1 = std::min(nch, c0 + b->piece);
+                for (int zt = 0; zt < p.nz / 32; ++zt)
+                    out.push_back(make_int4(i, zt, c0 | c1 << 16, k | np << 16));
             }
         }
-        if (ranges) {
+        const int nblk = (int)std::min<size_t>(out.size(), (size_t)max_blk);
+        if (ranges && b->scheme == COSENU_FV) {
+            // block k takes entries k, k + nblk, ...
+            std::vector<int4> in;
+            in.swap(out);
+            ranges->resize(nblk + 1);
+            for (int k = 0; k < nblk; ++k) {
+                (*ranges)[k] = (int)out.size();
+                for (size_t t = k; t < in.size(); t += nblk) out.push_back(in[t]);
+            }
+            (*ranges)[nblk] = (int)out.size();
+        } else if (ranges) {
             long long total = 0;
             for (long long x : w) total += x;
             ranges->assign(nblk + 1, (int)out.size());
@@ -163,11 +193,9 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
 {
     std::vector<int4> tab;
     std::vector<int> ranges;
-    size_t ntiles_all = 0;
-    for (int i : active) ntiles_all += b->m[i]->p.nz / 32;
     const int per_sm = b->use_tma ? tma_blocks_per_sm(b->scheme) : 1;
-    const int nblk = (int)std::min<size_t>(std::max<size_t>(ntiles_all, 1), (size_t)(per_sm * b->nsm));
-    size_t nt = build_table(b, active, tab, &ranges, nblk);
+    size_t nt = build_table(b, active, tab, &ranges, per_sm * b->nsm);
+    const int nblk = (int)ranges.size() - 1;  // (TMA family)
     if (nt == 0 || nsteps <= 0) return COSENU_OK;
     // table entries, then (TMA family) the nblk + 1 block range starts
     const size_t nrange_int4 = b->use_tma ? (ranges.size() + 3) / 4 : 0;
@@ -182,7 +210,7 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
     BCK(cudaEventRecord(b->table_ev[k], b->stream));
     BatchDev bd0{b->d_table[k], (int)nt, b->d_args, b->d_maps,
                  reinterpret_cast<const int *>(b->d_table[k] + nt)};
-    if (getenv("COSENU_BATCH_RR")) bd0.range = nullptr;
+    if (b->scheme == COSENU_FD && getenv("COSENU_BATCH_RR")) bd0.range = nullptr;
     int max_nvz = 0;
     for (int i : active) max_nvz = std::max(max_nvz, b->m[i]->p.nvz);
     const StageArgs a0 = ctx_stage_args(b->m[active[0]], 1);
@@ -203,12 +231,14 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
         }
         return cudaSuccess;
     };
-    // one graph of up to 16 steps for this phase, replayed (FP32-bulk: an even
-    // number of steps, so that every replay starts from the same parity)
-    int chunk = (int)std::min<long long>(16, nsteps);
-    if (b->fp32 && chunk > 1) chunk &= ~1;
+    // Long phases: one graph of 16 steps, replayed (an even number, so that every
+    // replay starts from the same parity).  Short ones are launched directly: a
+    // capture costs about 0.5 ms of host time, as much as 45 steps of four
+    // launches, and held up runs of many short phases (16 members, 14 phases of a
+    // few steps: 7 of 10 ms).
+    const int chunk = 16;
     cudaGraphExec_t ge = nullptr;
-    {
+    if (nsteps >= 8 * chunk) {
         cudaStream_t cs;
         BCK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         cudaGraph_t g = nullptr;
@@ -226,16 +256,15 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
     }
     long long left = nsteps;
     cudaError_t e = cudaSuccess;
-    while (left >= chunk && e == cudaSuccess) {
+    while (ge && left >= chunk && e == cudaSuccess) {
         e = cudaGraphLaunch(ge, b->stream);
         left -= chunk;
-        if (chunk & 1) par ^= b->fp32;  // (an odd chunk is a single replay)
     }
     while (left-- > 0 && e == cudaSuccess) {
         e = launch_step(b->stream, par);
         par ^= b->fp32;
     }
-    b->graphs.push_back(ge);  // released once the stream has drained
+    if (ge) b->graphs.push_back(ge);  // released once the stream has drained
     if (e != cudaSuccess) return bfail(b, COSENU_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     for (int i : active) {
         b->m[i]->steps += nsteps;
@@ -301,6 +330,23 @@ int cosenu_batch_create(int n, const cosenu_params *params, cosenu_batch **out)
         cosenu_set_stream(b->m[i], b->stream);
         b->max_nvz = std::max(b->max_nvz, params[i].nvz);
         b->tv[i] = std::min(params[i].nvz, 64);
+    }
+    // FV: the piece height (chunks) for which dealing all members' entries out
+    // over the block slots takes the fewest chunk times, at a third of a chunk of
+    // overhead per entry
+    double best = 1e300;
+    const long long slots = (long long)tma_blocks_per_sm(b->scheme) * b->nsm;
+    const int max_piece = (b->max_nvz + 7) / 8;
+    for (int pc = 1, piece = 1; pc <= max_piece; ++pc) {
+        b->piece = pc;
+        long long items = 0;
+        for (int i = 0; i < n; ++i) items += (long long)(params[i].nz / 32) * fv_pieces(b, i);
+        const double c = (double)((items + slots - 1) / slots) * (pc + 1.0 / 3.0);
+        if (c < best) {
+            best = c;
+            piece = pc;
+        }
+        if (pc == max_piece) b->piece = piece;
     }
     if (cudaMalloc(&b->d_args, 8 * (size_t)n * sizeof(StageArgs)) != cudaSuccess ||
         cudaMalloc(&b->d_maps, 2 * NMAP_B * (size_t)n * sizeof(CUtensorMap)) != cudaSuccess ||

@@ -91,16 +91,19 @@ void choose_tile(cosenu_ctx *ctx, int layout = 0)
     const char *kenv = getenv("COSENU_KERNEL");
     bool force_ldg = kenv && std::string(kenv) == "ldg";
     bool force_tma = kenv && std::string(kenv) == "tma";
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p.device);
-    if (p.nz % 32 == 0 && p.nvz <= tma_max_nvz() &&
-        (layout == 1 || ((p.nz / 32 >= nsm || force_tma) && p.tile_z == 0 && p.tile_v == 0 &&
-                         !force_ldg))) {
-        // TMA path (grids with at least one 32-cell z tile per SM): tiles span all rows
+    cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, p.device);
+    const int nsm = ctx->nsm;
+    // TMA path.  FV: every grid up to tma_max_nvz() rows (its blocks share tiles
+    // and its last tile may be partial).  FD: grids with at least one 32-cell z
+    // tile per SM.
+    const bool fits = p.nvz <= tma_max_nvz() && (p.nz % 32 == 0 || (p.scheme == FV && layout == 0));
+    const bool wanted = p.scheme == FV || p.nz / 32 >= nsm || force_tma;
+    if (fits && (layout == 1 || (wanted && p.tile_z == 0 && p.tile_v == 0 && !force_ldg))) {
         ctx->use_tma = true;
         ctx->tz = 32;
         ctx->tv = p.nvz;
-        ctx->nvt = 1;
+        if (p.scheme == FV && layout == 0) ctx->tv = fv_piece_rows(p.nz, p.nvz, nsm);
+        ctx->nvt = (p.nvz + ctx->tv - 1) / ctx->tv;
         return;
     }
     int tz = p.tile_z;
@@ -192,8 +195,10 @@ cudaError_t launch_stage(cosenu_ctx *ctx, int stage, cudaStream_t s)
     StageArgs a = stage_args(ctx, stage, -1);
     cudaError_t e;
     if (ctx->use_tma) {
-        int nblk = std::min(ctx->p.nz / tma_box_tile(),
-                            tma_blocks_per_sm(ctx->p.scheme) * ctx->nsm);
+        const int nblk = ctx->p.scheme == FV
+                             ? fv_blocks(ctx->p.nz, ctx->nvt, ctx->nsm)
+                             : std::min(ctx->p.nz / tma_box_tile(),
+                                        tma_blocks_per_sm(ctx->p.scheme) * ctx->nsm);
         const CUtensorMap *mX, *mY, *mA, *mB;
         if (!ctx->fp32) {
             // stage 3 reads U at its own cells in the A slot
@@ -223,17 +228,20 @@ cudaError_t launch_stage(cosenu_ctx *ctx, int stage, cudaStream_t s)
 // kernel expired (the results of that launch are not to be trusted).  The
 // word stays set, and every later check reports it, until a new state is
 // uploaded or initialised (prepare_state clears it).
+int report_err_flag(cosenu_ctx *ctx, int h)
+{
+    if (!ctx->use_tma || h == 0) return COSENU_OK;
+    ctx->err = "stage kernel pipeline wait timed out (code " + std::to_string(h) + ")";
+    return COSENU_ERR_CUDA;
+}
+
 int check_err_flag(cosenu_ctx *ctx)
 {
     if (!ctx->use_tma) return COSENU_OK;
     int h = 0;
     CK(cudaMemcpyAsync(&h, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (h != 0) {
-        ctx->err = "stage kernel pipeline wait timed out (code " + std::to_string(h) + ")";
-        return COSENU_ERR_CUDA;
-    }
-    return COSENU_OK;
+    return report_err_flag(ctx, h);
 }
 
 cudaError_t launch_steps(cosenu_ctx *ctx, int n, cudaStream_t s)
@@ -282,9 +290,15 @@ int prepare_state(cosenu_ctx *ctx)
     if (ctx->err_flag) CK(cudaMemsetAsync(ctx->err_flag, 0, sizeof(int), ctx->stream));
     CK(launch_ghost_fill(ctx->Y, ctx->cs, ctx->ld, ctx->p.nz, ctx->p.nvz, ctx->H, ctx->p.bc,
                          ctx->stream));
-    if (ctx->p.flags & COSENU_COLL)
+    if (ctx->p.flags & COSENU_COLL) {
+        // (all of a tile's moments in its first piece)
+        if (ctx->mom_nvt_cap > ctx->nvt)
+            CK(cudaMemsetAsync(ctx->M[2], 0,
+                               (size_t)ctx->mom_nvt_cap * NMOM * ctx->p.nz * sizeof(double),
+                               ctx->stream));
         CK(launch_moments(ctx->Y, ctx->M[2], ctx->vz, ctx->cs, ctx->ld, ctx->p.nz, ctx->p.nvz,
                           ctx->tz, ctx->tv, ctx->stream));
+    }
     ctx->have_state = true;
     ctx->next_stage = 0;
     return COSENU_OK;
@@ -428,6 +442,7 @@ int ctx_create(const cosenu_params *pp, cosenu_ctx **out, int layout)
     const size_t ustate = ctx->fp32 ? state / 2 : state;  // U0, U1 (and U2: FP32-bulk)
     // ensemble members may later be re-tiled down to 8-row v tiles
     ctx->mom_nvt_cap = layout == 1 ? (p.nvz + 7) / 8 : ctx->nvt;
+    if (ctx->use_tma) ctx->mom_nvt_cap = std::max(ctx->mom_nvt_cap, (p.nvz + MAX_TV - 1) / MAX_TV);
     const size_t mom = (size_t)ctx->mom_nvt_cap * NMOM * p.nz * sizeof(double);
 #define AL(ptr, n)                                                              \
     if ((rc = alloc(ctx, (void **)&(ptr), (n))) != COSENU_OK) {                 \
@@ -506,14 +521,16 @@ int ctx_create(const cosenu_params *pp, cosenu_ctx **out, int layout)
         if (!r && ctx->U2)
             r = make_state_map(&ctx->mU2_40, ctx->U2, ub, ctx->ld, p.nvz, ctx->cs, bxu, rn);
         if (!ctx->U2) ctx->mU2_40 = ctx->mU1_40;  // unused in FP64
-        if (!r && tma_prepare() != cudaSuccess) r = -2;
+        if (!r && tma_prepare(p.scheme, ctx->fp32, p.fd_advec != 0 || p.ko_order == 5) != cudaSuccess)
+            r = -2;
         if (r) {
             // no tensor-map support: fall back to the register-tiled kernel
+            // (mom_nvt_cap has room for its v tiles)
             ctx->use_tma = false;
-            ctx->p.tile_z = ctx->p.tile_v = 0;
-            choose_tile(ctx);
+            ctx->tz = p.nz % 32 == 0 ? 32 : (p.nz % 16 == 0 ? 16 : 8);
+            ctx->tv = std::min(p.nvz, MAX_TV);
+            ctx->nvt = (p.nvz + ctx->tv - 1) / ctx->tv;
         }
-        cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, p.device);
     }
     const char *ng = getenv("COSENU_NO_GRAPH");
     ctx->use_graphs = !(ng && ng[0] == '1');
@@ -870,8 +887,12 @@ int cosenu_analyse(cosenu_ctx *ctx, cosenu_diag *out)
     CK(launch_diag(ctx->Y, ctx->S0, ctx->G, ctx->bG, ctx->cs, ctx->ld, ctx->p.nz, ctx->p.nvz,
                    ctx->dz, ctx->dv, ctx->diag_part, ctx->diag_out, ctx->stream));
     CK(cudaMemcpyAsync(ctx->h_pinned, ctx->diag_out, 13 * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->h_pinned + 13, ctx->err_flag, sizeof(int), cudaMemcpyDeviceToHost,
+                       ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (int rc = check_err_flag(ctx)) return rc;
+    int err = 0;
+    std::memcpy(&err, ctx->h_pinned + 13, sizeof(int));
+    if (int rc = report_err_flag(ctx, err)) return rc;
     const double *r = ctx->h_pinned;
     out->dP_max = r[0];
     out->avdP = r[1];

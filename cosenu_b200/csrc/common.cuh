@@ -49,8 +49,9 @@ struct StageArgs {
 };
 
 // Ensemble launch: one stage launch covers every active instance.  Entry t of
-// `table` names (instance, z tile, v tile, rows: nvz in the TMA family); `args` holds the four stage
-// arguments of every instance and `maps` its six tensor maps (Y and U0/U1
+// `table` names (instance, z tile, v tile, -) in the register-tiled family,
+// (instance, z tile, -, rows) in FD's TMA kernel and (instance, z tile, chunks,
+// moment pieces) in FV's (stage_fv.cu); `args` holds the four stage arguments of every instance and `maps` its six tensor maps (Y and U0/U1
 // input boxes; Y, A and U0 tile boxes).
 struct BatchDev {
     const int4 *table;

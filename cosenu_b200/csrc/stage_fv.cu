@@ -1,10 +1,11 @@
-// TMA-pipelined RK4 stage kernel of the FV scheme (WENO7, src/rhs_fv.hpp:115-236)
-// for grids with at least one 32-cell z tile per SM and for ensembles.
+// TMA-pipelined RK4 stage kernel of the FV scheme (WENO7, src/rhs_fv.hpp:115-236),
+// for single simulations of any size and for ensembles.
 //
 // Same arithmetic and epilogue as rk4_stage_kernel (stage.cu); what changes is
-// how the work reaches the SM.  Each block is persistent over z tiles of 32
-// cells that span all nvz rows.  Chunks of 8 rows x (32 + 2*4) cells of all 8
-// components of the stage input, and the matching cells of the operands the
+// how the work reaches the SM.  A block is persistent over work items, each a
+// run of 8-row chunks of a 32-cell z tile (Seg; the last tile of a row may be
+// partial).  Chunks of 8 rows x (32 + 2*4)
+// cells of all 8 components of the stage input, and the matching cells of the operands the
 // combine reads, stream into a ring of NBUF shared-memory buffers with
 // cp.async.bulk.tensor (one 3-D tensor-map copy per operand and chunk); eight
 // warps take one row each.  There is no producer warp: the last warp to
@@ -34,6 +35,15 @@
 // (cp.async at the start of the row, waited for after the face phase, which
 // hides the copy; loads into registers stalled the face phase's own loads).
 //
+// A single simulation's tiles are cut along v into pieces of equal height
+// (fv_piece_rows) where whole tiles would leave block slots empty; each item
+// writes the moments of its piece, and the next stage sums a tile's pieces in
+// order.  Items are dealt out along z within a v band, so that the blocks
+// running together read neighbouring cells of the same rows: an even split into
+// contiguous runs of chunks kept the slots fuller but read 256-byte fragments
+// all over the state (nz 65536 x nvz 512: stage 1 1.62 -> 1.75 ms, stage 3
+// 2.23 -> 2.80 ms).
+//
 // Every wait is bounded in time (globaltimer, limit StageArgs::wait_ns): on
 // expiry the kernel records a code in *err and carries on along the same
 // control path, so no barrier is left waiting and the host reports the error.
@@ -41,6 +51,7 @@
 // release count never completes and no warp refills it; before the block
 // exits one thread waits (bounded again) for the copies in flight, so no block
 // ends while a bulk copy still writes into its shared memory.
+#include <algorithm>
 #include <cstdlib>
 
 #include "tma.cuh"
@@ -139,6 +150,32 @@ __device__ __forceinline__ void load12(const float *p, float *x)
     }
 }
 
+// One run of chunks of a tile: chunks [c0, c1) of z tile zt of member inst, the
+// tile's moments in np pieces, this run the piece-th.
+struct Seg {
+    int inst, zt, c0, c1, piece, np;
+};
+
+// Item i of a single simulation: z tile i % nzt of v band i / nzt.
+__device__ __forceinline__ Seg seg_of(int i, const StageArgs &a, int nzt)
+{
+    Seg s;
+    s.inst = 0;
+    s.piece = i / nzt;
+    s.zt = i - s.piece * nzt;
+    s.np = a.nvt;
+    const int pc = a.tv / R;
+    s.c0 = s.piece * pc;
+    s.c1 = min(s.c0 + pc, (a.nvz + R - 1) / R);
+    return s;
+}
+
+// Ensemble table entry (batch.cu): member, z tile, c0 | c1 << 16, piece | np << 16.
+__device__ __forceinline__ Seg seg_of(const int4 e)
+{
+    return Seg{e.x, e.y, e.z & 0xffff, e.z >> 16, e.w & 0xffff, e.w >> 16};
+}
+
 }  // namespace fv
 
 // TIN: type of the streamed stage input (FP64: the stage value U or Y;
@@ -178,39 +215,57 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
     int *s_last = reinterpret_cast<int *>(s_cnt + NBUF);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nzt = BATCHED ? bd.ntiles : a0.nz / TZ;
-    // this block's tiles: a contiguous range of the ensemble table, or every
-    // gridDim.x-th z tile (table entry); its chunks in order (each tile in
-    // chunks of R rows): chunk ch of tile t is the block's n-th, and its
-    // copies go into buffer n % NBUF
-    const bool rr = !BATCHED || bd.range == nullptr;
-    const int t_first = rr ? blockIdx.x : bd.range[blockIdx.x];
-    const int t_end = rr ? nzt : bd.range[blockIdx.x + 1];
-    const int t_step = rr ? gridDim.x : 1;
-    auto nch_of = [&](int t) { return ((BATCHED ? bd.table[t].w : a0.nvz) + R - 1) / R; };
-    auto issue_at = [&](int t, int ch, uint32_t n) {
+    // this block's items: every gridDim.x-th of a single simulation, or a run of
+    // the ensemble table; chunk ch of the item at position p is the block's n-th
+    // chunk, and its copies go into buffer n % NBUF
+    const int nzt = (a0.nz + TZ - 1) / TZ;
+    int p_first = blockIdx.x, p_end = BATCHED ? 0 : nzt * a0.nvt;
+    const int p_step = BATCHED ? 1 : gridDim.x;
+    auto seg_at = [&](int p) {
+        if constexpr (BATCHED) return fv::seg_of(bd.table[p]);
+        else return fv::seg_of(p, a0, nzt);
+    };
+    auto issue_at = [&](const fv::Seg &s, int ch, uint32_t n) {
         if (a0.stall) return;
         const int b = n % NBUF;
         if constexpr (BATCHED) {
-            const int4 e = bd.table[t];
-            const CUtensorMap *m = &bd.maps[e.x * NMAP];
+            const CUtensorMap *m = &bd.maps[s.inst * NMAP];
             fv::issue_chunk<L>(smem + b * L::BUF, &full[b], &m[MI::X], &m[MI::Y], &m[MI::A],
-                               e.y * TZ, ch * R);
+                               s.zt * TZ, ch * R);
         } else {
-            fv::issue_chunk<L>(smem + b * L::BUF, &full[b], &mX, &mY, &mA, t * TZ, ch * R);
+            fv::issue_chunk<L>(smem + b * L::BUF, &full[b], &mX, &mY, &mA, s.zt * TZ, ch * R);
         }
         s_last[b] = (int)n;
     };
-    // (t, ch) moved k chunks on; false past the block's last tile
-    auto advance = [&](int &t, int &ch, int k) -> bool {
+    // (p, s, ch) moved k chunks on; false past the block's last segment
+    auto advance = [&](int &p, fv::Seg &s, int &ch, int k) -> bool {
         for (; k > 0; --k) {
-            if (++ch == nch_of(t)) {
-                ch = 0;
-                t += t_step;
-                if (t >= t_end) return false;
+            if (++ch == s.c1) {
+                p += p_step;
+                if (p >= p_end) return false;
+                s = seg_at(p);
+                ch = s.c0;
             }
         }
         return true;
+    };
+    // moment m of cell zz of a segment's tile: its pieces in order
+    auto moment_in = [&](const fv::Seg &s, int m, int zz) {
+        const StageArgs &a = BATCHED ? bd.args[s.inst * 4 + STAGE - 1] : a0;
+        double x = 0.0;
+        if ((a.flags & F_COLL) && s.zt * TZ + zz < a.nz) {
+            const double *q = a.Min + (long long)m * a.nz + s.zt * TZ + zz;
+            const long long st = (long long)NMOM * a.nz;
+            x = q[0];
+            for (int k = 1; k < s.np; k += 8) {  // eight loads in flight
+                double y[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] = k + j < s.np ? q[(k + j) * st] : 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x += y[j];
+            }
+        }
+        return x;
     };
 
     if (tid == 0) {
@@ -221,21 +276,33 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
             s_last[b] = -1;
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        int t = t_first, ch = 0;
-        if (t < t_end)
-            for (uint32_t n = 0; n < (uint32_t)NBUF; ++n) {
-                issue_at(t, ch, n);
-                if (!advance(t, ch, 1)) break;
-            }
     }
-    // moments of the stage input for the first tile
-    if (t_first < t_end && tid < NMOM * TZ) {
-        int inst, zt;
-        tma_tile<BATCHED>(bd, t_first, inst, zt);
-        const StageArgs &a = BATCHED ? bd.args[inst * 4 + STAGE - 1] : a0;
-        if (a.flags & F_COLL)
-            s_mom[tid / TZ][tid % TZ] = a.Min[(long long)(tid / TZ) * a.nz + zt * TZ + tid % TZ];
+    if constexpr (BATCHED) {
+        p_first = bd.range[blockIdx.x];
+        p_end = bd.range[blockIdx.x + 1];
     }
+    fv::Seg cur{0, 0, 0, 0, 0, 0};
+    if (p_first < p_end) cur = seg_at(p_first);
+    double vz_l = 0.0, fac_l = 0.0;  // row values, see the chunk loop
+    auto load_rows = [&](const StageArgs &a, int ch) {
+        const int vl = min((ch + lane) * R + warp, a.nvz - 1);
+        vz_l = __ldg(&a.vz[vl]);
+        fac_l = __ldg(&a.rowfac[vl]);
+    };
+    if (!BATCHED) load_rows(a0, cur.c0);
+    if (tid == 0 && p_first < p_end) {
+        int p = p_first;
+        fv::Seg s = cur;
+        int ch = s.c0;
+        for (uint32_t n = 0; n < (uint32_t)NBUF; ++n) {
+            issue_at(s, ch, n);
+            if (!advance(p, s, ch, 1)) break;
+        }
+    }
+    // moments of the stage input for the first tile (not by the issuing warp)
+    static_assert(NMOM < R, "one warp per moment, after warp 0");
+    if (p_first < p_end && warp >= 1 && warp <= NMOM)
+        s_mom[warp - 1][lane] = moment_in(cur, warp - 1, lane);
     __syncthreads();
 
     // face phase: this lane's quad of cells and its component (of four per
@@ -246,18 +313,15 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
 
     uint32_t it = 0;
     int s_inst = -1;  // member whose arguments s_args holds
-    int4 cur = make_int4(0, 0, 0, 0);
-    if (BATCHED && t_first < t_end) cur = bd.table[t_first];
-    for (int t = t_first; t < t_end; t += t_step) {
-        const int inst = BATCHED ? cur.x : 0, zt = BATCHED ? cur.y : t;
-        const int tn = t + t_step;
-        int4 nxt = cur;
-        if (BATCHED && tn < t_end) nxt = bd.table[tn];  // next tile's entry, one tile ahead
+    for (int p = p_first; p < p_end;) {
+        const int inst = cur.inst;
+        const int pn = p + p_step;
+        const fv::Seg nxt = pn < p_end ? seg_at(pn) : cur;
         if (BATCHED && inst != s_inst) {
             // a new member: its arguments into shared memory.  Read from there
             // (like a0 from parameter space) they cost no registers across the
             // chunk loop and cannot alias the stores to U and A.  The previous
-            // tile's epilogue ended with a barrier.
+            // segment's epilogue ended with a barrier.
             if (tid < (int)(sizeof(StageArgs) / 8))
                 reinterpret_cast<long long *>(s_args)[tid] =
                     reinterpret_cast<const long long *>(&bd.args[inst * 4 + STAGE - 1])[tid];
@@ -265,43 +329,36 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
             s_inst = inst;
         }
         const StageArgs &a = BATCHED ? *s_args : a0;
-        const int nch = (a.nvz + R - 1) / R;
         const bool coll = (a.flags & F_COLL) != 0;
         const bool advec = (a.flags & F_ADVEC_OFF) == 0;
         const bool open_bc = a.bc != 0;
-        const int z0 = zt * TZ;
+        const int z0 = cur.zt * TZ;
         const int z = z0 + lane;
-        // prefetch the next tile's input moments into a register
+        const bool inz = z < a.nz;  // (the last tile of a row may be partial)
+        // the next segment's input moments, in a register until the epilogue
+        const bool new_tile = nxt.inst != inst || nxt.zt != cur.zt;
         double mnext = 0.0;
-        if (tid < NMOM * TZ && tn < t_end) {
-            const int in2 = BATCHED ? nxt.x : 0, zn = BATCHED ? nxt.y : tn;
-            const StageArgs &an = BATCHED ? bd.args[in2 * 4 + STAGE - 1] : a0;
-            if (an.flags & F_COLL)
-                mnext = an.Min[(long long)(tid / TZ) * an.nz + zn * TZ + tid % TZ];
-        }
-        // this warp's moment slots (the previous tile's epilogue has read them)
+        if (tid < NMOM * TZ && new_tile) mnext = moment_in(nxt, tid / TZ, tid % TZ);
+        // this warp's moment slots (the previous segment's epilogue has read them)
 #pragma unroll
         for (int m = 0; m < NMOM; ++m) s_red[warp][m][lane] = 0.0;
 
-        double vz_l = 0.0, fac_l = 0.0;
-        // only the first and last tile of a row hold cells that ghosts copy
-        const bool has_ghosts = z0 == 0 || z0 + TZ == a.nz;
+        if (BATCHED || p != p_first) load_rows(a, cur.c0);  // (the first: above)
+        // only tiles at a row's ends hold cells that ghosts copy
+        const bool has_ghosts = z0 == 0 || z0 + TZ > a.nz - a.H;
 
-        for (int ch = 0; ch < nch; ++ch, ++it) {
+        for (int ch = cur.c0; ch < cur.c1; ++ch, ++it) {
             const int b = it % NBUF;
             const int v = ch * R + warp;
             const bool valid = v < a.nvz;
             const int vr = valid ? v : a.nvz - 1;
             const long long ro = (long long)vr * a.ld + HP;
             // this row's velocity and advection factor from the host tables:
-            // lane l holds those of the warp's row in chunk ch - ch % 32 + l
-            if (ch % 32 == 0) {
-                const int vl = min((ch + lane) * R + warp, a.nvz - 1);
-                vz_l = __ldg(&a.vz[vl]);
-                fac_l = __ldg(&a.rowfac[vl]);
-            }
-            const double vzv = __shfl_sync(0xffffffffu, vz_l, ch % 32);
-            const double factor = __shfl_sync(0xffffffffu, fac_l, ch % 32);
+            // lane l holds those of the warp's row l chunks after chunk c0 + 32 k
+            const int cl = (ch - cur.c0) % 32;
+            if (cl == 0 && ch != cur.c0) load_rows(a, ch);
+            const double vzv = __shfl_sync(0xffffffffu, vz_l, cl);
+            const double factor = __shfl_sync(0xffffffffu, fac_l, cl);
             if constexpr (L::OWNED) {
                 // the combine's own operands, for after the face phase
                 unsigned char *own = s_own + warp * fv::OWN;
@@ -476,7 +533,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                 o[BEXI] += (2.0 * ct * c[BEXR] + st * (c[BEE] - c[BXX])) * pmo;
             }
             if (a.flags & F_MAT) {
-                const double hm = a.Hm[z];
+                const double hm = a.Hm[min(z, a.nz - 1)];
                 o[EXR] += hm * c[EXI];
                 o[EXI] += -hm * c[EXR];
                 o[BEXR] += -hm * c[BEXI];
@@ -558,26 +615,29 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                 ring_release_count(&s_cnt[b]) == (it / NBUF) * R + (R - 1)) {
                 // the last of the R warps to release buffer b: its next chunk
                 fence_proxy_async_smem();
-                int t2 = t, ch2 = ch;
-                if (advance(t2, ch2, NBUF)) issue_at(t2, ch2, it + NBUF);
+                int p2 = p;
+                fv::Seg s2 = cur;
+                int ch2 = ch;
+                if (advance(p2, s2, ch2, NBUF)) issue_at(s2, ch2, it + NBUF);
             }
 
-            if (valid) {
+            if (valid) {  // (uniform over the warp)
                 TOUT *row = static_cast<TOUT *>(a.U) + ro;
 #pragma unroll
                 for (int q = 0; q < NCOMP; ++q) {
-                    row[q * a.cs + z] = u[q];
-                    if (!INC && STAGE == 3) a.A[q * a.cs + ro + z] = anew[q];
+                    if (inz) {
+                        row[q * a.cs + z] = u[q];
+                        if (!INC && STAGE == 3) a.A[q * a.cs + ro + z] = anew[q];
+                    }
                 }
                 if (has_ghosts) {
 #pragma unroll
                     for (int q = 0; q < NCOMP; ++q) {
                         if (!open_bc) {
                             if (z < a.H) row[q * a.cs + z + a.nz] = u[q];
-                            if (z >= a.nz - a.H) row[q * a.cs + z - a.nz] = u[q];
+                            if (z >= a.nz - a.H && inz) row[q * a.cs + z - a.nz] = u[q];
                             continue;
                         }
-                        // (valid is uniform over the warp)
                         TOUT p0 = __shfl_sync(0xffffffffu, u[q], lane > 0 ? lane - 1 : 0);
                         if (z == 0)
                             for (int g = 1; g <= a.H; ++g) row[q * a.cs - g] = u[q];
@@ -592,7 +652,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                         }
                     }
                 }
-                if (coll) {
+                if (coll && inz) {
                     const double Am = um[EXI] + um[BEXI];
                     const double Bm = um[EXR] - um[BEXR];
                     const double Cm = um[EE] - um[XX] - um[BEE] + um[BXX];
@@ -605,8 +665,8 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                 }
             }
         }
-        // tile epilogue: output moments (fixed-order sum over warps) and the
-        // next tile's input moments
+        // segment epilogue: its output moments (fixed-order sum over warps) and
+        // the next segment's input moments
         if (coll || BATCHED) {
             __syncthreads();
             if (tid < NMOM * TZ) {
@@ -614,11 +674,13 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                 double s = 0.0;
 #pragma unroll
                 for (int w = 0; w < R; ++w) s += s_red[w][m][zz];
-                if (coll) a.Mout[(long long)m * a.nz + z0 + zz] = s;
-                s_mom[m][zz] = mnext;  // every warp read this tile's values above
+                if (coll && z0 + zz < a.nz)
+                    a.Mout[(long long)(cur.piece * NMOM + m) * a.nz + z0 + zz] = s;
+                if (new_tile) s_mom[m][zz] = mnext;  // every warp read this tile's values above
             }
             __syncthreads();
         }
+        p = pn;
         cur = nxt;
     }
     // the last copies issued into each buffer have landed before the block
@@ -647,6 +709,33 @@ static int minb_env()
 
 int fv_blocks_per_sm() { return minb_env(); }
 int fv_box_x(int elem_bytes) { return elem_bytes == 8 ? fv::xw<double>() : fv::xw<float>(); }
+
+// Rows of a v piece of a single simulation's tiles: the height (a multiple of
+// 8) for which the rounds of items over the block slots take the fewest
+// chunk times, at half a chunk of overhead per item.
+int fv_piece_rows(int nz, int nvz, int nsm)
+{
+    const int nzt = (nz + tma::TZ - 1) / tma::TZ, nch = (nvz + fv::R - 1) / fv::R;
+    const int slots = minb_env() * nsm;
+    int best = nch;
+    double cost = 1e300;
+    for (int nvt = 1; nvt <= nch; ++nvt) {
+        const int pc = (nch + nvt - 1) / nvt;
+        const long long items = (long long)nzt * ((nch + pc - 1) / pc);
+        const double c = (double)((items + slots - 1) / slots) * (pc + 0.5);
+        if (c < cost) {
+            cost = c;
+            best = pc;
+        }
+    }
+    return best * fv::R;
+}
+
+int fv_blocks(int nz, int nvt, int nsm)
+{
+    return (int)std::min<long long>((long long)((nz + tma::TZ - 1) / tma::TZ) * nvt,
+                                    (long long)minb_env() * nsm);
+}
 
 template <int STAGE, class TIN, class TOUT, int NB, int MINB>
 static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *err, int nblocks,
@@ -682,11 +771,6 @@ static cudaError_t launch_one(const tma::StageMaps &m, const StageArgs &a, int *
     constexpr int NB2 = L::smem(4) <= lim ? 4 : (L::smem(3) <= lim ? 3 : 2);
     static_assert(L::smem(2) <= lim, "two blocks per SM");
     constexpr int NB1 = L::smem(4) <= TMA_SMEM_MAX ? 4 : 3;
-    if (nblocks <= 0) {
-        cudaError_t e = launch_nb<STAGE, TIN, TOUT, NB1, 1>(m, a, err, 0, s, bd);
-        if (e == cudaSuccess) e = launch_nb<STAGE, TIN, TOUT, NB2, 2>(m, a, err, 0, s, bd);
-        return e;
-    }
     if (minb_env() == 1) return launch_nb<STAGE, TIN, TOUT, NB1, 1>(m, a, err, nblocks, s, bd);
     return launch_nb<STAGE, TIN, TOUT, NB2, 2>(m, a, err, nblocks, s, bd);
 }

@@ -609,15 +609,6 @@ static cudaError_t launch_one(const tma::StageMaps &m, const StageArgs &a, int *
                               cudaStream_t s, const BatchDev *bd)
 {
 #define LNB(NB, MINB) launch_nb<GEN, STAGE, TIN, TOUT, NB, MINB>(m, a, err, nblocks, s, bd)
-    if (nblocks <= 0) {
-        cudaError_t e = LNB(2, 1);
-        if (e == cudaSuccess) e = LNB(3, 1);
-        if (e == cudaSuccess) e = LNB(4, 1);
-        if (e == cudaSuccess) e = LNB(2, 2);
-        if (e == cudaSuccess) e = LNB(3, 2);
-        if (e == cudaSuccess) e = LNB(4, 2);
-        return e;
-    }
     if (tma_minb_fd_env() == 2) {
         const int lim = tma_smem_limit(2);
         if (tma_smem<TIN, TOUT, STAGE>(4) <= lim) return LNB(4, 2);
@@ -684,21 +675,18 @@ cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, i
     return launch_any(m, a, scheme, stage, fp32, err, nblocks, s, &bd);
 }
 
-// Sets the shared-memory attribute of every instantiation on the current device.
-cudaError_t tma_prepare()
+// Sets the shared-memory attribute of the kernels a simulation (or ensemble) of
+// this variant launches, on the current device.
+cudaError_t tma_prepare(int scheme, int fp32, bool gen)
 {
     CUtensorMap m{};
     StageArgs a{};
-    for (int sch = 0; sch < 2; ++sch)
-        for (int gen = 0; gen < 2; ++gen)
-            for (int fp32 = 0; fp32 < 2; ++fp32)
-                for (int st = 1; st <= 4; ++st) {
-                    a.fd_advec = gen;
-                    a.ko_order = 3;
-                    cudaError_t e = launch_rk4_stage_tma(m, m, m, m, a, sch, st, fp32, nullptr, 0,
-                                                         nullptr);
-                    if (e != cudaSuccess) return e;
-                }
+    a.fd_advec = gen;
+    a.ko_order = 3;
+    for (int st = 1; st <= 4; ++st) {
+        cudaError_t e = launch_rk4_stage_tma(m, m, m, m, a, scheme, st, fp32, nullptr, 0, nullptr);
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 

@@ -44,7 +44,11 @@ def _compare(oracle, case, precision, steps=3, seed=0, **kw):
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("bc", ["periodic", "open"])
-@pytest.mark.parametrize("nz,nvz", [(32, 1), (32, 7), (64, 8), (64, 9), (96, 33), (160, 264)])
+# partial last tiles of 8, 16 and 24 cells (down to a lone one), tiles shared by
+# as many blocks as they have chunks, and (968, 77): 310 chunks on 296 block
+# slots, so that blocks straddle tiles
+@pytest.mark.parametrize("nz,nvz", [(32, 1), (32, 7), (64, 8), (64, 9), (96, 33), (160, 264),
+                                    (16, 3), (24, 8), (40, 17), (72, 9), (968, 77)])
 def test_fv_pipelined_kernel_edges(gpu_lib, oracle, monkeypatch, nz, nvz, bc, precision):
     from oracle.oracle import Case
     monkeypatch.setenv("COSENU_KERNEL", "tma")
