@@ -20,6 +20,8 @@
 #include <vector>
 
 #include "../../include/cosenu_b200.h"
+#include "mlp_math.cuh"
+#include "mlp_train.h"
 
 cudaError_t mlp_gemm_tc(const __nv_bfloat16 *A, long long sam, long long sak,
                         const __nv_bfloat16 *B, long long sbk, long long sbn, int M, int N, int K,
@@ -39,13 +41,8 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi)
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
-__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-
-__device__ __forceinline__ float gelu_grad(float x)
-{
-    return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) +
-           x * 0.39894228040143268f * expf(-0.5f * x * x);
-}
+using mlpmath::gelu;
+using mlpmath::gelu_grad;
 
 __global__ void __launch_bounds__(128) gemm_bf16_kernel(
     const __nv_bfloat16 *__restrict__ A, long long sam, long long sak,
@@ -188,21 +185,12 @@ __global__ void colsum_kernel(const float *dZ, int M, int N, float *db)
 
 // AdamW on FP32 master parameters; refreshes the BF16 copy of weights.
 __global__ void adamw_kernel(float *w, const float *g, float *m, float *v, __nv_bfloat16 *wb,
-                             long long n, float lr, float b1, float b2, float eps, float wd,
-                             float c1, float c2)
+                             long long n, mlpmath::AdamW p, float wd)
 {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float gi = g[i];
-    float mi = b1 * m[i] + (1.f - b1) * gi;
-    float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    float mh = mi / c1, vh = vi / c2;
-    float wi = w[i];
-    wi -= lr * (mh / (sqrtf(vh) + eps) + wd * wi);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16(wi);
+    mlpmath::adamw(w[i], m[i], v[i], g[i], p, wd);
+    if (wb) wb[i] = __float2bfloat16(w[i]);
 }
 
 __global__ void to_bf16_kernel(const float *x, __nv_bfloat16 *y, long long n)
@@ -254,6 +242,13 @@ struct cosenu_mlp {
     __nv_bfloat16 *dAb = nullptr;
     float *T = nullptr, *partial = nullptr;  // partial: 1024 floats, then eacc
     double *eacc = nullptr;                   // epoch loss sum, on the device
+    // fused training: gradients per layer, an epoch's rows in shuffled order,
+    // loss partials of every step
+    std::vector<__nv_bfloat16 *> dz;
+    int dz_cap = 0;
+    __nv_bfloat16 *xe = nullptr;
+    float *te = nullptr, *lossp = nullptr;
+    size_t xe_cap = 0, te_cap = 0, lossp_cap = 0;
     // resident training data
     float *dX = nullptr, *dT = nullptr;
     int *didx = nullptr;
@@ -399,6 +394,40 @@ int ensure_cap(cosenu_mlp *net, int rows)
     return COSENU_OK;
 }
 
+// Buffers of the fused training path: `batch` rows per step, ndata rows and
+// nsteps steps per epoch.
+int ensure_fused(cosenu_mlp *net, int batch, int nsteps)
+{
+    auto grow = [&](void **p, size_t &cap, size_t n) -> int {
+        if (n <= cap) return COSENU_OK;
+        cudaStreamSynchronize(net->stream);
+        if (*p) cudaFree(*p);
+        *p = nullptr;
+        cap = 0;
+        MCK(cudaMalloc(p, n));
+        cap = n;
+        return COSENU_OK;
+    };
+    int rc;
+    if ((rc = grow((void **)&net->xe, net->xe_cap, (size_t)net->ndata * net->kpad * 2)) ||
+        (rc = grow((void **)&net->te, net->te_cap, (size_t)net->ndata * net->nout * 4)) ||
+        (rc = grow((void **)&net->lossp, net->lossp_cap,
+                   (size_t)nsteps * mlptrain::loss_tiles(net->nout) * 4)))
+        return rc;
+    if (batch > net->dz_cap) {
+        cudaStreamSynchronize(net->stream);
+        for (auto &p : net->dz) {
+            if (p) cudaFree(p);
+            p = nullptr;
+        }
+        net->dz_cap = 0;
+        net->dz.resize(net->nl, nullptr);
+        for (int l = 0; l < net->nl; ++l) MCK(cudaMalloc(&net->dz[l], (size_t)batch * net->dout[l] * 2));
+        net->dz_cap = batch;
+    }
+    return COSENU_OK;
+}
+
 // forward over `rows` rows already in net->xb; output pre-activation of the
 // last layer in Z[nl-1]
 void forward(cosenu_mlp *net, int rows)
@@ -528,12 +557,14 @@ int cosenu_mlp_destroy(cosenu_mlp *net)
     if (net->stream) cudaStreamSynchronize(net->stream);
     void *bufs[] = {net->w, net->g, net->m1, net->m2, net->wb, net->partial, net->xb, net->dA,
                     net->dB, net->dAb, net->T, net->dX, net->dT, net->didx, net->dxin, net->dtin,
-                    net->derr};
+                    net->derr, net->xe, net->te, net->lossp};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (auto p : net->Z)
         if (p) cudaFree(p);
     for (auto p : net->Hb)
+        if (p) cudaFree(p);
+    for (auto p : net->dz)
         if (p) cudaFree(p);
     collect_times(net);
     for (cudaEvent_t e : net->ev_pool) cudaEventDestroy(e);
@@ -655,6 +686,34 @@ int cosenu_mlp_train(cosenu_mlp *net, int epochs, int batch, float lr, float wei
     uint64_t st = shuffle_seed * 6364136223846793005ull + 1442695040888963407ull;
     const int nb = 32;
     double esum = 0;
+    const mlpmath::AdamW opt0{lr, beta1, beta2, eps, weight_decay, 0.f, 0.f};
+    // The fused kernels (mlp_train.cu) where they take the network and batch; the
+    // timing mode needs the separate launches it brackets by class.
+    const int nsteps = (net->ndata + batch - 1) / batch, tiles = mlptrain::loss_tiles(net->nout);
+    const bool fused = net->tc && !net->timing &&
+                       mlptrain::fits(net->nl, net->din.data(), net->dout.data(), batch);
+    std::vector<float> lossp;
+    mlptrain::Args fa{};
+    if (fused) {
+        if ((rc = ensure_fused(net, batch, nsteps)) != COSENU_OK) return rc;
+        MCK(mlptrain::prepare());
+        lossp.resize((size_t)nsteps * tiles);
+        fa.nl = net->nl;
+        fa.w = net->w;
+        fa.m1 = net->m1;
+        fa.m2 = net->m2;
+        fa.wb = net->wb;
+        fa.err = net->derr;
+        for (int l = 0; l < net->nl; ++l) {
+            fa.din[l] = net->din[l];
+            fa.dout[l] = net->dout[l];
+            fa.woff[l] = net->woff[l];
+            fa.boff[l] = net->boff[l];
+            fa.z[l] = net->Z[l];
+            fa.h[l] = net->Hb[l];
+            fa.dz[l] = net->dz[l];
+        }
+    }
     for (int e = 0; e < epochs; ++e) {
         for (int i = 0; i < net->ndata; ++i) perm[i] = i;
         for (int i = net->ndata - 1; i > 0; --i) {  // Fisher-Yates
@@ -666,8 +725,27 @@ int cosenu_mlp_train(cosenu_mlp *net, int epochs, int batch, float lr, float wei
                             net->stream));
         MCK(cudaMemsetAsync(net->eacc, 0, sizeof(double), net->stream));
         long long ecount = 0;
+        if (fused)  // the epoch's rows in BF16, in shuffled order
+            gather_kernel<<<net->ndata, 128, 0, net->stream>>>(net->dX, net->dT, net->didx,
+                                                               net->ndata, net->nin, net->kpad,
+                                                               net->nout, net->xe, net->te);
         for (int b0 = 0; b0 < net->ndata; b0 += batch) {
             const int rows = std::min(batch, net->ndata - b0);
+            net->t_step++;
+            mlpmath::AdamW opt = opt0;
+            opt.c1 = 1.f - std::pow(beta1, (float)net->t_step);
+            opt.c2 = 1.f - std::pow(beta2, (float)net->t_step);
+            ecount += (long long)rows * net->nout;
+            if (fused) {
+                fa.rows = rows;
+                fa.x = net->xe + (size_t)b0 * net->kpad;
+                fa.t = net->te + (size_t)b0 * net->nout;
+                fa.scale = 1.f / ((float)rows * net->nout);
+                fa.loss = net->lossp + (size_t)(b0 / batch) * tiles;
+                fa.opt = opt;
+                MCK(mlptrain::step(fa, net->stream));
+                continue;
+            }
             {
                 Timed tm(net, K_ELEM);
                 gather_kernel<<<rows, 128, 0, net->stream>>>(net->dX, net->dT, net->didx + b0,
@@ -676,28 +754,30 @@ int cosenu_mlp_train(cosenu_mlp *net, int epochs, int batch, float lr, float wei
             }
             forward(net, rows);
             backward(net, rows, nb);
-            net->t_step++;
-            const float c1 = 1.f - std::pow(beta1, (float)net->t_step);
-            const float c2 = 1.f - std::pow(beta2, (float)net->t_step);
             Timed *tm = new Timed(net, K_ADAMW);
             for (int l = 0; l < net->nl; ++l) {
                 const long long nw = (long long)net->din[l] * net->dout[l];
                 adamw_kernel<<<(unsigned)((nw + 255) / 256), 256, 0, net->stream>>>(
                     net->w + net->woff[l], net->g + net->woff[l], net->m1 + net->woff[l],
-                    net->m2 + net->woff[l], net->wb + net->woff[l], nw, lr, beta1, beta2, eps,
-                    weight_decay, c1, c2);
+                    net->m2 + net->woff[l], net->wb + net->woff[l], nw, opt, weight_decay);
                 adamw_kernel<<<(net->dout[l] + 255) / 256, 256, 0, net->stream>>>(
                     net->w + net->boff[l], net->g + net->boff[l], net->m1 + net->boff[l],
-                    net->m2 + net->boff[l], net->wb + net->boff[l], net->dout[l], lr, beta1, beta2,
-                    eps, 0.f, c1, c2);
+                    net->m2 + net->boff[l], net->wb + net->boff[l], net->dout[l], opt, 0.f);
             }
             delete tm;  // the AdamW updates of all layers
             loss_accumulate_kernel<<<1, 32, 0, net->stream>>>(net->partial, nb, net->eacc);
-            ecount += (long long)rows * net->nout;
         }
         // one host synchronisation per epoch (the shuffle buffer is reused)
-        MCK(cudaMemcpyAsync(&esum, net->eacc, sizeof(double), cudaMemcpyDeviceToHost, net->stream));
+        if (fused)
+            MCK(cudaMemcpyAsync(lossp.data(), net->lossp, lossp.size() * 4, cudaMemcpyDeviceToHost,
+                                net->stream));
+        else
+            MCK(cudaMemcpyAsync(&esum, net->eacc, sizeof(double), cudaMemcpyDeviceToHost, net->stream));
         MCK(cudaStreamSynchronize(net->stream));
+        if (fused) {
+            esum = 0;
+            for (float x : lossp) esum += x;
+        }
         collect_times(net);
         if ((rc = check_device(net)) != COSENU_OK) return rc;
         if (epoch_loss) epoch_loss[e] = (float)(esum / ecount);

@@ -31,6 +31,8 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "mlp_math.cuh"
+
 namespace mlpgemm {
 
 constexpr int TBM = 128;  // rows of the tile = TMEM lanes
@@ -118,7 +120,7 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo)
            ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
 }
 
-__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
+using mlpmath::gelu;
 
 __device__ __forceinline__ uint32_t word(const uint4 &v, int w)
 {

@@ -296,7 +296,9 @@ int cosenu_mlp_train(cosenu_mlp *net, int epochs, int batch, float lr, float wei
  * its device time added to one of three classes, read by cosenu_mlp_timing as
  * ms[0] GEMMs (forward, dX, dW), ms[1] elementwise kernels (gather, MSE,
  * GELU backward, bias column sums), ms[2] AdamW updates.  Setting the mode
- * clears the totals. */
+ * clears the totals.  While it is on, training runs these as separate launches;
+ * otherwise batches of up to 512 rows go through fused kernels that give the
+ * same parameters bit for bit. */
 int cosenu_mlp_set_timing(cosenu_mlp *net, int on);
 int cosenu_mlp_timing(const cosenu_mlp *net, double ms[3]);
 
