@@ -90,19 +90,18 @@ void choose_tile(cosenu_ctx *ctx, int layout = 0)
     const cosenu_params &p = ctx->p;
     const char *kenv = getenv("COSENU_KERNEL");
     bool force_ldg = kenv && std::string(kenv) == "ldg";
-    bool force_tma = kenv && std::string(kenv) == "tma";
     cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, p.device);
     const int nsm = ctx->nsm;
-    // TMA path.  FV: every grid up to tma_max_nvz() rows (its blocks share tiles
-    // and its last tile may be partial).  FD: grids with at least one 32-cell z
-    // tile per SM.
-    const bool fits = p.nvz <= tma_max_nvz() && (p.nz % 32 == 0 || (p.scheme == FV && layout == 0));
-    const bool wanted = p.scheme == FV || p.nz / 32 >= nsm || force_tma;
-    if (fits && (layout == 1 || (wanted && p.tile_z == 0 && p.tile_v == 0 && !force_ldg))) {
+    // TMA path: every grid up to tma_max_nvz() rows (tiles are cut along v where
+    // there are too few of them, and the last one of a row may be partial)
+    const bool fits = p.nvz <= tma_max_nvz() && (p.nz % 32 == 0 || layout == 0);
+    if (fits && (layout == 1 || (p.tile_z == 0 && p.tile_v == 0 && !force_ldg))) {
         ctx->use_tma = true;
         ctx->tz = 32;
         ctx->tv = p.nvz;
-        if (p.scheme == FV && layout == 0) ctx->tv = fv_piece_rows(p.nz, p.nvz, nsm);
+        if (layout == 0)
+            ctx->tv = p.scheme == FV ? fv_piece_rows(p.nz, p.nvz, nsm)
+                                     : fd_piece_rows(p.nz, p.nvz, ctx->fp32, nsm);
         ctx->nvt = (p.nvz + ctx->tv - 1) / ctx->tv;
         return;
     }
@@ -195,10 +194,7 @@ cudaError_t launch_stage(cosenu_ctx *ctx, int stage, cudaStream_t s)
     StageArgs a = stage_args(ctx, stage, -1);
     cudaError_t e;
     if (ctx->use_tma) {
-        const int nblk = ctx->p.scheme == FV
-                             ? fv_blocks(ctx->p.nz, ctx->nvt, ctx->nsm)
-                             : std::min(ctx->p.nz / tma_box_tile(),
-                                        tma_blocks_per_sm(ctx->p.scheme) * ctx->nsm);
+        const int nblk = tma_blocks(ctx->p.scheme, ctx->p.nz, ctx->nvt, ctx->nsm);
         const CUtensorMap *mX, *mY, *mA, *mB;
         if (!ctx->fp32) {
             // stage 3 reads U at its own cells in the A slot

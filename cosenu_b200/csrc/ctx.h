@@ -25,7 +25,8 @@ int tma_box_tile();
 int tma_max_nvz();
 int tma_blocks_per_sm(int scheme);
 int fv_piece_rows(int nz, int nvz, int nsm);
-int fv_blocks(int nz, int nvt, int nsm);
+int fd_piece_rows(int nz, int nvz, int fp32, int nsm);
+int tma_blocks(int scheme, int nz, int nvt, int nsm);
 cudaError_t tma_prepare(int scheme, int fp32, bool gen);
 cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
                                  const CUtensorMap &mA, const CUtensorMap &mB, const StageArgs &a,

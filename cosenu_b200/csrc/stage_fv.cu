@@ -344,9 +344,6 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
         for (int m = 0; m < NMOM; ++m) s_red[warp][m][lane] = 0.0;
 
         if (BATCHED || p != p_first) load_rows(a, cur.c0);  // (the first: above)
-        // only tiles at a row's ends hold cells that ghosts copy
-        const bool has_ghosts = z0 == 0 || z0 + TZ > a.nz - a.H;
-
         for (int ch = cur.c0; ch < cur.c1; ++ch, ++it) {
             const int b = it % NBUF;
             const int v = ch * R + warp;
@@ -630,28 +627,6 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                         if (!INC && STAGE == 3) a.A[q * a.cs + ro + z] = anew[q];
                     }
                 }
-                if (has_ghosts) {
-#pragma unroll
-                    for (int q = 0; q < NCOMP; ++q) {
-                        if (!open_bc) {
-                            if (z < a.H) row[q * a.cs + z + a.nz] = u[q];
-                            if (z >= a.nz - a.H && inz) row[q * a.cs + z - a.nz] = u[q];
-                            continue;
-                        }
-                        TOUT p0 = __shfl_sync(0xffffffffu, u[q], lane > 0 ? lane - 1 : 0);
-                        if (z == 0)
-                            for (int g = 1; g <= a.H; ++g) row[q * a.cs - g] = u[q];
-                        if (z == a.nz - 1) {
-                            TOUT p1 = u[q];
-                            for (int g = 0; g < a.H; ++g) {
-                                TOUT gh = p1 * TOUT(2) - p0;
-                                row[q * a.cs + a.nz + g] = gh;
-                                p0 = p1;
-                                p1 = gh;
-                            }
-                        }
-                    }
-                }
                 if (coll && inz) {
                     const double Am = um[EXI] + um[BEXI];
                     const double Bm = um[EXR] - um[BEXR];
@@ -664,6 +639,13 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                     s_red[warp][5][lane] += vzv * Cm;
                 }
             }
+        }
+        // ghost cells (written by the cells' own lanes in the chunk loop, periodic
+        // ones too cost every tile: nz 65536 x nvz 512 7.33 -> 7.70 ms a step)
+        if (z0 == 0 || z0 + TZ > a.nz - a.H) {
+            __syncthreads();
+            fill_ghosts<true>(static_cast<TOUT *>(a.U), a, cur.c0 * R, min(cur.c1 * R, a.nvz), z0, tid,
+                        fv::NTHR);
         }
         // segment epilogue: its output moments (fixed-order sum over warps) and
         // the next segment's input moments
@@ -729,12 +711,6 @@ int fv_piece_rows(int nz, int nvz, int nsm)
         }
     }
     return best * fv::R;
-}
-
-int fv_blocks(int nz, int nvt, int nsm)
-{
-    return (int)std::min<long long>((long long)((nz + tma::TZ - 1) / tma::TZ) * nvt,
-                                    (long long)minb_env() * nsm);
 }
 
 template <int STAGE, class TIN, class TOUT, int NB, int MINB>

@@ -2,8 +2,11 @@
 // FV scheme's is stage_fv.cu.
 //
 // Same arithmetic and epilogue as rk4_stage_kernel (stage.cu); what changes
-// is how the operands reach the SM.  Each block is persistent over z-tiles of
-// 32 cells that span all nvz rows.  One producer warp streams chunks of 8 (or
+// is how the operands reach the SM.  Each block is persistent over work items:
+// z tiles of 32 cells (the last of a row may be partial) that span all nvz
+// rows, or v bands of them where whole tiles would leave SMs idle
+// (fd_piece_rows; an item then writes the moments of its band, and the next
+// stage sums a tile's bands in order).  One producer warp streams chunks of 8 (or
 // 12) rows x (32 + 2*4) cells of all 8 components of the stage input, and the
 // matching cells of Y and A, into a ring of NBUF shared-memory buffers with
 // cp.async.bulk.tensor (one 3-D tensor-map copy per operand and chunk, box
@@ -25,6 +28,7 @@
 // producer's next wait on that buffer fails too and it stops issuing copies;
 // before the block exits it waits (bounded again) for the copies in flight, so
 // no block ends while a bulk copy still writes into its shared memory.
+#include <algorithm>
 #include <cstdlib>
 
 #include "tma.cuh"
@@ -91,6 +95,11 @@ __device__ __forceinline__ void issue_chunk(unsigned char *buf, uint64_t *bar, c
 
 }  // namespace tma
 
+// Work item: z tile zt of member inst, rows [v0, v1), v band vt of nvt.
+struct FdItem {
+    int inst, zt, v0, v1, vt, nvt;
+};
+
 // FD: velocity and advection factor of row i, recomputed with round-to-nearest
 // operations so the bits equal the host tables (capi.cu, src/nuosc.hpp:88-92,
 // rhs_fd.hpp:57).  The FD stages are bound by memory latency, and a table load
@@ -104,6 +113,47 @@ __device__ __forceinline__ void fd_row_values(double v0, double dv, double dz, i
     if (fd_advec == 0) f = __ddiv_rn(-v, d12);                      // centre
     else if (fd_advec == 1) f = __ddiv_rn(__dmul_rn(-sv, v), d12);  // upwind
     else f = __ddiv_rn(__dmul_rn(sv, v), d12);                       // lopsided
+}
+
+// Weights of one row's combined advection (src/rhs_fd.hpp:53-73) and
+// Kreiss-Oliger (:128-145) stencil for the neighbours -1 .. -T, then +1 .. +T
+// (T = 2: central FD4 + KO3; T = 3: any).  One difference and one multiply-add
+// per neighbour; the separate stencils, with the upwind side indexed by sign(v)
+// and a branch per component and variant, took 96-99 us a step on 4000 x 100
+// cells where the central one took 69.
+template <bool GEN>
+__device__ __forceinline__ void fd_weights(const StageArgs &a, double v, double f, double *w)
+{
+    const double e = a.ko_eps;
+    if constexpr (!GEN) {
+        w[0] = -8.0 * f - 4.0 * e;
+        w[1] = f + e;
+        w[2] = 8.0 * f - 4.0 * e;
+        w[3] = e - f;
+    } else {
+        const bool k5 = a.ko_order == 5;
+        const double e1 = k5 ? 15.0 * e : -4.0 * e, e2 = k5 ? -6.0 * e : e, e3 = k5 ? e : 0.0;
+        if (a.fd_advec == 0) {
+            w[0] = e1 - 8.0 * f;
+            w[1] = e2 + f;
+            w[2] = e3;
+            w[3] = e1 + 8.0 * f;
+            w[4] = e2 - f;
+            w[5] = e3;
+        } else {
+            // weights of the upwind neighbours 1 .. 3 and the downwind one
+            const bool up = a.fd_advec == 1;
+            const double u1 = e1 + (up ? -36.0 : 18.0) * f, u2 = e2 + (up ? 18.0 : -6.0) * f,
+                         u3 = e3 + (up ? -4.0 : 1.0) * f, d1 = e1 + (up ? 0.0 : -3.0) * f;
+            const bool left = v > 0.0;  // (v = 0: f = 0, both sides alike)
+            w[0] = left ? u1 : d1;
+            w[1] = left ? u2 : e2;
+            w[2] = left ? u3 : e3;
+            w[3] = left ? d1 : u1;
+            w[4] = left ? e2 : u2;
+            w[5] = left ? e3 : u3;
+        }
+    }
 }
 
 // TIN: type of the streamed stage input (FP64: the stage value U or Y;
@@ -131,7 +181,24 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
     double(*s_red)[NMOM][TZ] = reinterpret_cast<double(*)[NMOM][TZ]>(s_mom + NMOM);  // [NRED]
     StageArgs *s_args = reinterpret_cast<StageArgs *>(s_red + L::NRED);  // batched: current member
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nzt = BATCHED ? bd.ntiles : a0.nz / TZ;
+    // a single simulation's items: all z tiles of a v band, then the next band's
+    const int nzt = BATCHED ? 1 : (a0.nz + TZ - 1) / TZ;
+    const int nitems = BATCHED ? bd.ntiles : nzt * a0.nvt;
+    auto item_at = [&](int t) {
+        FdItem i;
+        if constexpr (BATCHED) {
+            const int4 e = bd.table[t];  // (member, z tile, -, rows)
+            i = FdItem{e.x, e.y, 0, e.w, 0, 1};
+        } else {
+            i.inst = 0;
+            i.vt = t / nzt;
+            i.zt = t - i.vt * nzt;
+            i.nvt = a0.nvt;
+            i.v0 = i.vt * a0.tv;
+            i.v1 = min(i.v0 + a0.tv, a0.nvz);
+        }
+        return i;
+    };
 
     if (tid == 0) {
         for (int b = 0; b < NBUF; ++b) {
@@ -149,27 +216,26 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
             bool issuing = true;  // false once a wait has failed: no further copies
             const bool rr = !BATCHED || bd.range == nullptr;  // interleaved tiles
             const int t_first = rr ? blockIdx.x : bd.range[blockIdx.x];
-            const int t_end = rr ? nzt : bd.range[blockIdx.x + 1];
+            const int t_end = rr ? nitems : bd.range[blockIdx.x + 1];
             const int t_step = rr ? gridDim.x : 1;
-            // batched: table entries (member, z tile, -, nvz) are read one tile
-            // ahead, and a new member's tensor maps (global memory) are
-            // prefetched while the previous tile streams
-            int4 cur = make_int4(0, 0, 0, 0);
-            if (BATCHED && t_first < t_end) cur = bd.table[t_first];
+            // items are read one ahead, and (batched) a new member's tensor maps
+            // (global memory) are prefetched while the previous tile streams
+            FdItem cur{};
+            if (t_first < t_end) cur = item_at(t_first);
             for (int t = t_first; t < t_end && issuing; t += t_step) {
                 const bool has_next = t + t_step < t_end;
-                int4 nxt = cur;
-                if (BATCHED && has_next) nxt = bd.table[t + t_step];
-                const int inst = BATCHED ? cur.x : 0, zt = BATCHED ? cur.y : t;
+                FdItem nxt = cur;
+                if (has_next) nxt = item_at(t + t_step);
+                const int inst = cur.inst;
                 const CUtensorMap *px = BATCHED ? &bd.maps[inst * NMAP + MI::X] : &mX;
                 const CUtensorMap *py = BATCHED ? &bd.maps[inst * NMAP + MI::Y] : &mY;
                 const CUtensorMap *pa = BATCHED ? &bd.maps[inst * NMAP + MI::A] : &mA;
                 const CUtensorMap *pb = BATCHED ? &bd.maps[inst * NMAP + MI::B] : &mB;
-                const int z0 = zt * TZ;
-                const int nch = ((BATCHED ? cur.w : a0.nvz) + R - 1) / R;
+                const int z0 = cur.zt * TZ;
+                const int nch = (cur.v1 - cur.v0 + R - 1) / R;
                 for (int ch = 0; ch < nch; ++ch, ++it) {
-                    if (BATCHED && ch == 0 && has_next && nxt.x != inst) {
-                        const CUtensorMap *m = &bd.maps[nxt.x * NMAP];
+                    if (BATCHED && ch == 0 && has_next && nxt.inst != inst) {
+                        const CUtensorMap *m = &bd.maps[nxt.inst * NMAP];
                         tma::prefetch_map(&m[MI::X]);
                         if (L::YB) tma::prefetch_map(&m[MI::Y]);
                         if (L::AB) tma::prefetch_map(&m[MI::A]);
@@ -181,7 +247,8 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                         issuing = false;  // a consumer gave up: buffer b may still be in use
                         break;
                     }
-                    issue_chunk<L>(smem + b * L::BUF, &full[b], px, py, pa, pb, z0, ch * R);
+                    issue_chunk<L>(smem + b * L::BUF, &full[b], px, py, pa, pb, z0,
+                                   cur.v0 + ch * R);
                 }
                 cur = nxt;
             }
@@ -194,31 +261,46 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
     }
 
     // ---------------------------------------------------------------- consumers
-    // this block's tiles: a contiguous range of the ensemble table, or every
-    // gridDim.x-th z tile of a single simulation
+    // this block's items: a contiguous range of the ensemble table, or every
+    // gridDim.x-th one of a single simulation
     const bool rr = !BATCHED || bd.range == nullptr;
     const int t_first = rr ? blockIdx.x : bd.range[blockIdx.x];
-    const int t_end = rr ? nzt : bd.range[blockIdx.x + 1];
+    const int t_end = rr ? nitems : bd.range[blockIdx.x + 1];
     const int t_step = rr ? gridDim.x : 1;
+    // moment m of cell zz of an item's tile: its bands in order
+    auto moment_in = [&](const FdItem &i, int m, int zz) {
+        const StageArgs &a = BATCHED ? bd.args[i.inst * 4 + STAGE - 1] : a0;
+        double x = 0.0;
+        if ((a.flags & F_COLL) && i.zt * TZ + zz < a.nz) {
+            const double *q = a.Min + (long long)m * a.nz + i.zt * TZ + zz;
+            const long long st = (long long)NMOM * a.nz;
+            x = q[0];
+            for (int k = 1; k < i.nvt; k += 8) {  // eight loads in flight
+                double y[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) y[j] = k + j < i.nvt ? q[(k + j) * st] : 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x += y[j];
+            }
+        }
+        return x;
+    };
+    FdItem ahead{};  // batched: the next table entry, read one item ahead
+    if (t_first < t_end) ahead = item_at(t_first);
     // moments of the stage input for the first tile
-    if (t_first < t_end && tid < NMOM * TZ) {
-        int inst, zt;
-        tma_tile<BATCHED>(bd, t_first, inst, zt);
-        const StageArgs &a = BATCHED ? bd.args[inst * 4 + STAGE - 1] : a0;
-        if (a.flags & F_COLL)
-            s_mom[tid / TZ][tid % TZ] = a.Min[(long long)(tid / TZ) * a.nz + zt * TZ + tid % TZ];
-    }
+    if (t_first < t_end && tid < NMOM * TZ)
+        s_mom[tid / TZ][tid % TZ] = moment_in(ahead, tid / TZ, tid % TZ);
     consumer_sync();
 
     uint32_t it = 0;
     int s_inst = -1;  // member whose arguments s_args holds
-    int4 cur = make_int4(0, 0, 0, 0);
-    if (BATCHED && t_first < t_end) cur = bd.table[t_first];
     for (int t = t_first; t < t_end; t += t_step) {
-        const int inst = BATCHED ? cur.x : 0, zt = BATCHED ? cur.y : t;
+        // (a single simulation's items are cheap to work out again, and their
+        // fields would hold registers across the chunk loop)
+        const FdItem cur = BATCHED ? ahead : item_at(t);
+        const int inst = cur.inst, v0 = cur.v0, v1 = cur.v1;
         const int tn = t + t_step;
-        int4 nxt = cur;
-        if (BATCHED && tn < t_end) nxt = bd.table[tn];  // next tile's entry, one tile ahead
+        if (BATCHED && tn < t_end) ahead = item_at(tn);
         if (BATCHED && inst != s_inst) {
             // a new member: its arguments into shared memory.  Read from there
             // (like a0 from parameter space) they cost no registers across the
@@ -231,26 +313,21 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
             s_inst = inst;
         }
         const StageArgs &a = BATCHED ? *s_args : a0;
-        const int nch = (a.nvz + R - 1) / R;
+        const int nch = (v1 - v0 + R - 1) / R;
         const bool coll = (a.flags & F_COLL) != 0;
         const bool advec = (a.flags & F_ADVEC_OFF) == 0;
-        const bool open_bc = a.bc != 0;
-        const int z0 = zt * TZ;
+        const int z0 = cur.zt * TZ;
         const int z = z0 + lane;
-        // prefetch the next tile's input moments into a register
+        // the next item's input moments, in a register until the epilogue
         double mnext = 0.0;
-        if (tid < NMOM * TZ && tn < t_end) {
-            const int in2 = BATCHED ? nxt.x : 0, zn = BATCHED ? nxt.y : tn;
-            const StageArgs &an = BATCHED ? bd.args[in2 * 4 + STAGE - 1] : a0;
-            if (an.flags & F_COLL)
-                mnext = an.Min[(long long)(tid / TZ) * an.nz + zn * TZ + tid % TZ];
-        }
+        if (tid < NMOM * TZ && tn < t_end) mnext = moment_in(BATCHED ? ahead : item_at(tn), tid / TZ, tid % TZ);
         double macc[NMOM] = {0, 0, 0, 0, 0, 0};
+        // only tiles at a row's ends hold cells that ghosts copy
+        const bool wrap = a.bc == 0 && (z0 == 0 || z0 + TZ > a.nz - a.H);
         for (int ch = 0; ch < nch; ++ch, ++it) {
             const int b = it % NBUF;
-            const int v = ch * R + warp;
-            const bool valid = v < a.nvz;
-            const int vr = valid ? v : a.nvz - 1;
+            const int v = v0 + ch * R + warp;
+            const int vr = min(v, a.nvz - 1);
             double vzv, factor;
             fd_row_values(a.v0, a.dv, a.dz, a.fd_advec, vr, vzv, factor);
             const bool landed = tma::mbar_wait(&full[b], (it / NBUF) & 1, err, 2, a0.wait_ns);
@@ -269,10 +346,10 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                     return (double)xrow[q * XW + j];
             };
 
-            double c[NCOMP], o[NCOMP], ko[NCOMP];
+            double c[NCOMP], o[NCOMP];
 #pragma unroll
             for (int q = 0; q < NCOMP; ++q) c[q] = in(q, lane);
-            // FD: vacuum, matter, advection, (collective below), dissipation
+            // vacuum, matter, advection and dissipation, (collective below)
 #pragma unroll
             for (int q = 0; q < NCOMP; ++q) o[q] = 0.0;
             if (a.flags & F_VAC) {
@@ -289,39 +366,43 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                 o[BEXI] = pmo * (2.0 * ct * c[BEXR] + st * (c[BEE] - c[BXX]));
             }
             if (a.flags & F_MAT) {
-                const double hm = a.Hm[z];
+                const double hm = a.Hm[min(z, a.nz - 1)];
                 o[EXR] += hm * c[EXI];
                 o[EXI] += -hm * c[EXR];
                 o[BEXR] += -hm * c[BEXI];
                 o[BEXI] += hm * c[BEXR];
             }
-            const int sv = (vzv > 0.0) - (vzv < 0.0);
-            const double ko_eps = a.ko_eps;
-            // one pass over each stencil: advection now, dissipation kept
-            // for after the collective term (the reference's order)
+            double ko[NCOMP];
+            if constexpr (!GEN && !INC) {
+                // FP64's central variant is bound by HBM and keeps the separate
+                // sums: advection now, dissipation after the collective term
+                const double ko_eps = a.ko_eps, fa = advec ? factor : 0.0;
 #pragma unroll
-            for (int q = 0; q < NCOMP; ++q) {
-                const double m2 = in(q, lane - 2), m1 = in(q, lane - 1), p1 = in(q, lane + 1),
-                             p2 = in(q, lane + 2);
-                if (advec) {
-                    double adv;
-                    if (!GEN || a.fd_advec == 0) {
-                        adv = factor * ((m2 - p2) - 8.0 * (m1 - p1));
-                    } else if (a.fd_advec == 1) {
-                        adv = factor * (-4.0 * in(q, lane - 3 * sv) + 18.0 * in(q, lane - 2 * sv) -
-                                        36.0 * in(q, lane - sv) + 22.0 * c[q]);
-                    } else {
-                        adv = factor * (in(q, lane - 3 * sv) - 6.0 * in(q, lane - 2 * sv) +
-                                        18.0 * in(q, lane - sv) - 10.0 * c[q] -
-                                        3.0 * in(q, lane + sv));
-                    }
-                    o[q] += adv;
-                }
-                if (GEN && a.ko_order == 5)
-                    ko[q] = ko_eps * (in(q, lane - 3) + in(q, lane + 3) - 6.0 * (m2 + p2) +
-                                      15.0 * (m1 + p1) - 20.0 * c[q]);
-                else
+                for (int q = 0; q < NCOMP; ++q) {
+                    const double m2 = in(q, lane - 2), m1 = in(q, lane - 1), p1 = in(q, lane + 1),
+                                 p2 = in(q, lane + 2);
+                    o[q] += fa * ((m2 - p2) - 8.0 * (m1 - p1));
                     ko[q] = ko_eps * (m2 + p2 - 4.0 * (m1 + p1) + 6.0 * c[q]);
+                }
+            } else {
+                // advection and dissipation as one stencil of differences from
+                // the centre (the weights of either sum to zero); FP32-bulk,
+                // latency bound at 128 registers: nz 32768 x nvz 256, stages 2
+                // and 3 0.276 -> 0.245 ms each
+                constexpr int TAPS = GEN ? 3 : 2;
+                double w[2 * TAPS];
+                fd_weights<GEN>(a, vzv, advec ? factor : 0.0, w);
+#pragma unroll
+                for (int q = 0; q < NCOMP; ++q) {
+                    double x = 0.0;
+#pragma unroll
+                    for (int k = 1; k <= TAPS; ++k) {
+                        x += w[k - 1] * (in(q, lane - k) - c[q]);
+                        x += w[TAPS + k - 1] * (in(q, lane + k) - c[q]);
+                    }
+                    o[q] += x;
+                    ko[q] = 0.0;
+                }
             }
             if (coll) {
                 // this tile's input moments, read where used (they stay in
@@ -341,9 +422,10 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                 o[BEXR] += mudv * ((c[BXX] - c[BEE]) * SA - c[BEXI] * SC);
                 o[BEXI] += mudv * ((c[BXX] - c[BEE]) * SB + c[BEXR] * SC);
             }
+            if constexpr (!GEN && !INC) {
 #pragma unroll
-            for (int q = 0; q < NCOMP; ++q) o[q] += ko[q];
-
+                for (int q = 0; q < NCOMP; ++q) o[q] += ko[q];
+            }
             // stage combine.  FP64 (stage values, A written once by stage 3 from
             // U in the A slot, U' and Y) or FP32-bulk (increments, common.cuh).
             const double dt = a.dt;
@@ -397,13 +479,7 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
             __syncwarp();
             if (lane == 0 && landed) tma::mbar_arrive(&empty[b]);
 
-            TOUT uleft[NCOMP];
-            if (open_bc) {
-#pragma unroll
-                for (int q = 0; q < NCOMP; ++q)
-                    uleft[q] = __shfl_sync(0xffffffffu, u[q], lane > 0 ? lane - 1 : 0);
-            }
-            if (valid) {
+            if (v < v1 && z < a.nz) {  // (the last tile may be partial)
                 TOUT *U = static_cast<TOUT *>(a.U);
                 const long long ro = (long long)v * a.ld + HP;
 #pragma unroll
@@ -411,22 +487,7 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                     TOUT *row = U + q * a.cs + ro;
                     row[z] = u[q];
                     if (!INC && STAGE == 3) a.A[q * a.cs + ro + z] = anew[q];
-                    if (!open_bc) {
-                        if (z < a.H) row[z + a.nz] = u[q];
-                        if (z >= a.nz - a.H) row[z - a.nz] = u[q];
-                    } else {
-                        if (z == 0)
-                            for (int g = 1; g <= a.H; ++g) row[-g] = u[q];
-                        if (z == a.nz - 1) {
-                            TOUT p0 = uleft[q], p1 = u[q];
-                            for (int g = 0; g < a.H; ++g) {
-                                TOUT gh = p1 * TOUT(2) - p0;
-                                row[a.nz + g] = gh;
-                                p0 = p1;
-                                p1 = gh;
-                            }
-                        }
-                    }
+                    if (wrap) periodic_ghosts(row, a, z, u[q]);
                 }
                 if (coll) {
                     const double Am = um[EXI] + um[BEXI];
@@ -441,8 +502,12 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                 }
             }
         }
-        // tile epilogue: output moments (fixed-order sum over warps) and the
-        // next tile's input moments
+        if (a.bc != 0 && (z0 == 0 || z0 + TZ >= a.nz)) {
+            consumer_sync();
+            fill_ghosts<false>(static_cast<TOUT *>(a.U), a, v0, v1, z0, tid, R * 32);
+        }
+        // item epilogue: output moments (fixed-order sum over warps) and the
+        // next item's input moments
         if (coll || BATCHED) {
             // warps w and w + R/2 pair up, then the R/2 pair sums are added
             // in a fixed order
@@ -461,12 +526,13 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
                 double s = 0.0;
 #pragma unroll
                 for (int w = 0; w < R / 2; ++w) s += s_red[w][m][zz];
-                if (coll) a.Mout[(long long)m * a.nz + z0 + zz] = s;
+                const int vt = BATCHED ? 0 : t / nzt;
+                if (coll && z0 + zz < a.nz)
+                    a.Mout[(long long)(vt * NMOM + m) * a.nz + z0 + zz] = s;
                 s_mom[m][zz] = mnext;  // every consumer read this tile's values above
             }
             consumer_sync();
         }
-        cur = nxt;
     }
 }
 
@@ -560,6 +626,29 @@ static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *e
     return cudaGetLastError();
 }
 
+// Rows of a v band of a single simulation's tiles: the height for which the
+// rounds of items over the SMs take the fewest chunk times, summed over the four
+// stages, at one chunk of overhead per item.
+int fd_piece_rows(int nz, int nvz, int fp32, int nsm)
+{
+    const int nzt = (nz + tma::TZ - 1) / tma::TZ;
+    const int r[4] = {12, fp32 ? 12 : 8, fp32 ? 12 : 8, 8};  // rows()
+    int best = nvz;
+    double cost = 1e300;
+    for (int nvt = 1; nvt <= (nvz + 3) / 4; ++nvt) {
+        const int tv = ((nvz + nvt - 1) / nvt + 3) / 4 * 4;
+        const long long items = (long long)nzt * ((nvz + tv - 1) / tv);
+        double c = 0.0;
+        for (int s = 0; s < 4; ++s) c += (tv + r[s] - 1) / r[s] + 1.0;
+        c *= (double)((items + nsm - 1) / nsm);
+        if (c < cost) {
+            cost = c;
+            best = std::min(tv, nvz);
+        }
+    }
+    return best;
+}
+
 // Ring depth of the FD kernel (one block per SM): the deepest ring of at most
 // 4 buffers that total at most 144 KB.  Measured at nz 32768 x nvz 256:
 // stages of 53-54 KB chunks (FP64 stage 3) are fastest with 2 buffers
@@ -603,6 +692,13 @@ static int tma_minb_fd_env()
 }
 
 int tma_blocks_per_sm(int scheme) { return scheme == FV ? fv_blocks_per_sm() : tma_minb_fd_env(); }
+
+// Blocks of a single simulation: every block slot, or one item each.
+int tma_blocks(int scheme, int nz, int nvt, int nsm)
+{
+    return (int)std::min<long long>((long long)((nz + tma::TZ - 1) / tma::TZ) * nvt,
+                                    (long long)tma_blocks_per_sm(scheme) * nsm);
+}
 
 template <bool GEN, int STAGE, class TIN, class TOUT>
 static cudaError_t launch_one(const tma::StageMaps &m, const StageArgs &a, int *err, int nblocks,

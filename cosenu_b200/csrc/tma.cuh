@@ -164,16 +164,61 @@ struct StageMaps {
 
 static_assert(sizeof(StageArgs) % 8 == 0, "StageArgs is copied to shared memory in 8-byte words");
 
-template <bool BATCHED>
-__device__ __forceinline__ void tma_tile(const BatchDev &bd, int t, int &inst, int &zt)
+// Ghost cells that hold output cell z of a tile under the periodic boundary
+// (updateBufferZone, src/nuosc.hpp:212-278), written by the cell's own lane; `row`
+// points at cell 0 of its row and component.
+template <class TOUT>
+__device__ __forceinline__ void periodic_ghosts(TOUT *row, const StageArgs &a, int z, TOUT u)
 {
-    if (BATCHED) {
-        const int4 e = bd.table[t];
-        inst = e.x;
-        zt = e.y;
-    } else {
-        inst = 0;
-        zt = t;
+    if (z < a.H) row[z + a.nz] = u;
+    if (z >= a.nz - a.H) row[z - a.nz] = u;
+}
+
+// Ghost cells of rows [v0, v1) that follow from a tile (at z0) at a row's end:
+// periodic copies, or the open boundary's first cell on the left and running
+// linear extrapolation on the right.  One thread per row and component, after a
+// barrier behind the stores of the tile's cells: under the open boundary, written
+// inside the chunk loop, one lane stored 4 cells of 8 components in turn while
+// the stage waited (FD, 4000 x 100 cells: 139 us a step against 69 under the
+// periodic one).  PERIODIC: the periodic copies too.
+template <bool PERIODIC, class TOUT>
+__device__ __forceinline__ void fill_ghosts(TOUT *U, const StageArgs &a, int v0, int v1, int z0,
+                                            int tid, int nthr)
+{
+    // cells [s, s + n) copied to [d, d + n), four loads in flight
+    auto copy = [](TOUT *row, int d, int s, int n) {
+        for (int g = 0; g < n; g += 4) {
+            TOUT x[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (g + k < n) x[k] = row[s + g + k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (g + k < n) row[d + g + k] = x[k];
+        }
+    };
+    const int zr = max(z0, a.nz - a.H);  // the tile's cells that wrap to the left
+#pragma unroll 2
+    for (int i = tid; i < (v1 - v0) * NCOMP; i += nthr) {
+        TOUT *row = U + (i % NCOMP) * a.cs + (long long)(v0 + i / NCOMP) * a.ld + HP;
+        if (PERIODIC && a.bc == 0) {
+            if (z0 == 0) copy(row, a.nz, 0, a.H);
+            copy(row, zr - a.nz, zr, min(z0 + tma::TZ, a.nz) - zr);
+        } else {
+            if (z0 == 0) {
+                const TOUT x = row[0];
+                for (int g = 1; g <= a.H; ++g) row[-g] = x;
+            }
+            if (z0 + tma::TZ >= a.nz) {
+                TOUT p0 = row[a.nz - 2], p1 = row[a.nz - 1];
+                for (int g = 0; g < a.H; ++g) {
+                    const TOUT x = p1 * TOUT(2) - p0;
+                    row[a.nz + g] = x;
+                    p0 = p1;
+                    p1 = x;
+                }
+            }
+        }
     }
 }
 

@@ -1,7 +1,8 @@
 """The pipelined stage kernels at the sizes where their tiling can go wrong:
 one tile (whose cells are copied to both ghost zones), row counts around the
 8-row chunk, rows of both signs of v in a chunk, both boundaries, on rough data
-(random differences of 0.1 between neighbours), against long double.
+(random differences of 0.1 between neighbours), against long double (FV) or the
+CPU oracle (FD).
 
 Tolerances.  FP64: the differences are rounding, a few 1e-16 per operation and
 stage; 1e-12 leaves four orders for three steps.  FP32-bulk: an increment
@@ -32,7 +33,10 @@ def _rough(case, oracle, seed):
 def _compare(oracle, case, precision, steps=3, seed=0, **kw):
     from tests._util import gpu_from_case
     st0 = _rough(case, oracle, seed)
-    ref = longdouble.step(case, st0[..., case.gz:case.gz + case.nz], steps)
+    if case.scheme == "fv":
+        ref = longdouble.step(case, st0[..., case.gz:case.gz + case.nz], steps)
+    else:
+        ref = oracle.step(case, st0, steps)
     with gpu_from_case(case, precision=precision, **kw) as sim:
         tile = sim.tile()
         sim.upload(st0)
@@ -54,4 +58,17 @@ def test_fv_pipelined_kernel_edges(gpu_lib, oracle, monkeypatch, nz, nvz, bc, pr
     monkeypatch.setenv("COSENU_KERNEL", "tma")
     case = Case(nz=nz, nvz=nvz, gz=4, z0=-nz / 4, z1=nz / 4, scheme="fv", bc=bc, omega=1e-2,
                 theta_deg=37.0, mat=True, mu=0.5)
+    assert _compare(oracle, case, precision)[0] == 32
+
+
+# FD: as above with its chunks of 8 and 12 rows, and bands of v (200 x 37: 7
+# tiles in bands of 12 rows; 1000 x 100: 32 tiles on 148 SMs)
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("bc,fd_advec,ko", [("periodic", "center", 3), ("open", "center", 3),
+                                            ("open", "lopsided", 5), ("periodic", "upwind", 5)])
+@pytest.mark.parametrize("nz,nvz", [(16, 1), (24, 13), (32, 8), (40, 25), (200, 37), (1000, 100)])
+def test_fd_pipelined_kernel_edges(gpu_lib, oracle, nz, nvz, bc, fd_advec, ko, precision):
+    from oracle.oracle import Case
+    case = Case(nz=nz, nvz=nvz, gz=4, z0=-nz / 4, z1=nz / 4, scheme="fd", bc=bc, omega=1e-2,
+                theta_deg=37.0, mat=True, mu=0.5, fd_advec=fd_advec, ko_order=ko)
     assert _compare(oracle, case, precision)[0] == 32
