@@ -39,6 +39,7 @@ def nvcc() -> str:
 def _headers() -> list[str]:
     return glob.glob(os.path.join(CSRC, "**", "*.cuh"), recursive=True) + \
         glob.glob(os.path.join(CSRC, "**", "*.hpp"), recursive=True) + \
+        glob.glob(os.path.join(CSRC, "**", "*.h"), recursive=True) + \
         glob.glob(os.path.join(INCLUDE, "*.h")) + glob.glob(os.path.join(INCLUDE, "*.hpp"))
 
 
