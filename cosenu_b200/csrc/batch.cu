@@ -216,7 +216,7 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
     const StageArgs a0 = ctx_stage_args(b->m[active[0]], 1);
     // the active members' common buffer parity (0 for FP64)
     int par = b->m[active[0]]->ypar;
-    auto launch_step = [&](cudaStream_t s, int p) -> cudaError_t {
+    auto launch_step = [&](cudaStream_t s, int p, bool chained) -> cudaError_t {
         BatchDev bd = bd0;
         bd.args += (size_t)p * 4 * b->n;
         bd.maps += (size_t)p * NMAP_B * b->n;
@@ -224,7 +224,7 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
             cudaError_t e;
             if (b->use_tma)
                 e = launch_rk4_stage_tma_batch(bd, a0, b->scheme, st, b->fp32, b->err_flag, nblk,
-                                               max_nvz, s);
+                                               max_nvz, s, chained || st > 1);
             else
                 e = launch_rk4_stage_batch(bd, b->scheme, st, b->tz, b->fp32, s);
             if (e != cudaSuccess) return e;
@@ -245,7 +245,7 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
         cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             cudaError_t le = cudaSuccess;
-            for (int i = 0; i < chunk && le == cudaSuccess; ++i) le = launch_step(cs, par ^ (i & 1));
+            for (int i = 0; i < chunk && le == cudaSuccess; ++i) le = launch_step(cs, par ^ (i & 1), i > 0);
             e = cudaStreamEndCapture(cs, &g);
             if (le != cudaSuccess) e = le;
         }
@@ -260,8 +260,9 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
         e = cudaGraphLaunch(ge, b->stream);
         left -= chunk;
     }
-    while (left-- > 0 && e == cudaSuccess) {
-        e = launch_step(b->stream, par);
+    for (bool chained = false; left-- > 0 && e == cudaSuccess;) {
+        e = launch_step(b->stream, par, chained);
+        chained = true;
         par ^= b->fp32;
     }
     if (ge) b->graphs.push_back(ge);  // released once the stream has drained

@@ -188,8 +188,9 @@ void flip(cosenu_ctx *ctx)
 }
 
 // Launches one stage; after stage 4 of the FP32-bulk form the state is in the
-// other buffer.
-cudaError_t launch_stage(cosenu_ctx *ctx, int stage, cudaStream_t s)
+// other buffer.  chained: the previous operation on s is a stage launch of the
+// same call (launch_after).
+cudaError_t launch_stage(cosenu_ctx *ctx, int stage, cudaStream_t s, bool chained)
 {
     StageArgs a = stage_args(ctx, stage, -1);
     cudaError_t e;
@@ -212,7 +213,7 @@ cudaError_t launch_stage(cosenu_ctx *ctx, int stage, cudaStream_t s)
             mB = &ctx->mU1_32;
         }
         e = launch_rk4_stage_tma(*mX, *mY, *mA, *mB, a, ctx->p.scheme, stage, ctx->fp32,
-                                 ctx->err_flag, nblk, s);
+                                 ctx->err_flag, nblk, s, chained);
     } else {
         e = launch_rk4_stage(a, ctx->p.scheme, stage, ctx->tz, ctx->fp32, s);
     }
@@ -244,7 +245,7 @@ cudaError_t launch_steps(cosenu_ctx *ctx, int n, cudaStream_t s)
 {
     for (int i = 0; i < n; ++i)
         for (int st = 1; st <= 4; ++st) {
-            cudaError_t e = launch_stage(ctx, st, s);
+            cudaError_t e = launch_stage(ctx, st, s, i > 0 || st > 1);
             if (e != cudaSuccess) return e;
         }
     return cudaSuccess;
@@ -517,7 +518,8 @@ int ctx_create(const cosenu_params *pp, cosenu_ctx **out, int layout)
         if (!r && ctx->U2)
             r = make_state_map(&ctx->mU2_40, ctx->U2, ub, ctx->ld, p.nvz, ctx->cs, bxu, rn);
         if (!ctx->U2) ctx->mU2_40 = ctx->mU1_40;  // unused in FP64
-        if (!r && tma_prepare(p.scheme, ctx->fp32, p.fd_advec != 0 || p.ko_order == 5) != cudaSuccess)
+        if (!r && tma_prepare(p.scheme, ctx->fp32, p.fd_advec != 0 || p.ko_order == 5,
+                              layout == 1) != cudaSuccess)
             r = -2;
         if (r) {
             // no tensor-map support: fall back to the register-tiled kernel
@@ -798,7 +800,7 @@ int cosenu_step_stage(cosenu_ctx *ctx, int stage)
     if (!ctx->have_state) return fail(ctx, COSENU_ERR_STATE, "no state uploaded");
     if (stage != ctx->next_stage) return fail(ctx, COSENU_ERR_STATE, "stages must run in order 0..3");
     DeviceGuard dg(ctx->p.device);
-    CK(launch_stage(ctx, stage + 1, ctx->stream));
+    CK(launch_stage(ctx, stage + 1, ctx->stream, false));
     ctx->next_stage = (stage + 1) % 4;
     if (ctx->next_stage == 0) ctx->steps++;
     return COSENU_OK;

@@ -27,14 +27,14 @@ int tma_blocks_per_sm(int scheme);
 int fv_piece_rows(int nz, int nvz, int nsm);
 int fd_piece_rows(int nz, int nvz, int fp32, int nsm);
 int tma_blocks(int scheme, int nz, int nvt, int nsm);
-cudaError_t tma_prepare(int scheme, int fp32, bool gen);
+cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched);
 cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
                                  const CUtensorMap &mA, const CUtensorMap &mB, const StageArgs &a,
                                  int scheme, int stage, int fp32, int *err, int nblocks,
-                                 cudaStream_t s);
+                                 cudaStream_t s, bool chained);
 cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, int scheme,
                                        int stage, int fp32, int *err, int nblocks, int max_nvz,
-                                       cudaStream_t s);
+                                       cudaStream_t s, bool chained);
 cudaError_t launch_rk4_stage_batch(const BatchDev &bd, int scheme, int stage, int tz, int fp32,
                                    cudaStream_t s);
 }  // namespace cosenu

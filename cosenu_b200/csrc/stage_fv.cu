@@ -269,6 +269,11 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
     };
 
     if (tid == 0) {
+        if constexpr (!BATCHED) {
+            prefetch_map(&mX);
+            if (L::YB) prefetch_map(&mY);
+            if (L::AB) prefetch_map(&mA);
+        }
         for (int b = 0; b < NBUF; ++b) {
             mbar_init(&full[b], 1);
             mbar_init(&ebar[b], NE * 32);
@@ -290,6 +295,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
         fac_l = __ldg(&a.rowfac[vl]);
     };
     if (!BATCHED) load_rows(a0, cur.c0);
+    previous_launch();  // (what is read above, no stage writes)
     if (tid == 0 && p_first < p_end) {
         int p = p_first;
         fv::Seg s = cur;
@@ -647,6 +653,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
             fill_ghosts<true>(static_cast<TOUT *>(a.U), a, cur.c0 * R, min(cur.c1 * R, a.nvz), z0, tid,
                         fv::NTHR);
         }
+        if (pn >= p_end) next_launch();  // (chain.cuh)
         // segment epilogue: its output moments (fixed-order sum over warps) and
         // the next segment's input moments
         if (coll || BATCHED) {
@@ -719,8 +726,9 @@ static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *e
 {
     auto kern = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, false, MINB>;
     auto kernb = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, true, MINB>;
-    if (nblocks <= 0) {  // preparation call: shared-memory limit and carveout
+    if (nblocks <= 0) {  // preparation call: shared-memory limit and carveout (bd: both kernels)
         for (auto k : {kern, kernb}) {
+            if (k == kernb && !bd) continue;
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  TMA_SMEM_MAX);
             if (e == cudaSuccess)
@@ -731,11 +739,8 @@ static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *e
         return cudaSuccess;
     }
     constexpr int shmem = fv::Layout<TIN, TOUT, STAGE>::smem(NB);
-    if (bd)
-        kernb<<<nblocks, fv::NTHR, shmem, s>>>(*m.x, *m.y, *m.a, a, err, *bd);
-    else
-        kern<<<nblocks, fv::NTHR, shmem, s>>>(*m.x, *m.y, *m.a, a, err, BatchDev{});
-    return cudaGetLastError();
+    return launch_after(m.chained, bd ? kernb : kern, nblocks, fv::NTHR, shmem, s, *m.x, *m.y, *m.a,
+                        a, err, bd ? *bd : BatchDev{});
 }
 
 template <int STAGE, class TIN, class TOUT>

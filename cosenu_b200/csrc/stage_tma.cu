@@ -201,6 +201,12 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
     };
 
     if (tid == 0) {
+        if constexpr (!BATCHED) {
+            tma::prefetch_map(&mX);
+            if (L::YB) tma::prefetch_map(&mY);
+            if (L::AB) tma::prefetch_map(&mA);
+            if (INC && L::AB) tma::prefetch_map(&mB);
+        }
         for (int b = 0; b < NBUF; ++b) {
             tma::mbar_init(&full[b], 1);
             tma::mbar_init(&empty[b], R);
@@ -208,6 +214,7 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    previous_launch();  // (all threads: the producer's copies, the consumers' loads and stores)
 
     if (warp == R) {
         // ------------------------------------------------------------ producer
@@ -506,6 +513,7 @@ __global__ void __launch_bounds__(tma::Layout<TIN, TOUT, STAGE>::NTHR, MINB)
             consumer_sync();
             fill_ghosts<false>(static_cast<TOUT *>(a.U), a, v0, v1, z0, tid, R * 32);
         }
+        if (tn >= t_end) next_launch();  // (chain.cuh)
         // item epilogue: output moments (fixed-order sum over warps) and the
         // next item's input moments
         if (coll || BATCHED) {
@@ -606,8 +614,9 @@ static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *e
 {
     auto kern = rk4_stage_tma_kernel<GEN, STAGE, TIN, TOUT, NB, false, MINB>;
     auto kernb = rk4_stage_tma_kernel<GEN, STAGE, TIN, TOUT, NB, true, MINB>;
-    if (nblocks <= 0) {  // preparation call: shared-memory limit and carveout
+    if (nblocks <= 0) {  // preparation call: shared-memory limit and carveout (bd: both kernels)
         for (auto k : {kern, kernb}) {
+            if (k == kernb && !bd) continue;
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  TMA_SMEM_MAX);
             if (e == cudaSuccess)
@@ -619,11 +628,8 @@ static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *e
     }
     const int shmem = tma_smem<TIN, TOUT, STAGE>(NB);
     constexpr int NT = tma::Layout<TIN, TOUT, STAGE>::NTHR;
-    if (bd)
-        kernb<<<nblocks, NT, shmem, s>>>(*m.x, *m.y, *m.a, *m.b, a, err, *bd);
-    else
-        kern<<<nblocks, NT, shmem, s>>>(*m.x, *m.y, *m.a, *m.b, a, err, BatchDev{});
-    return cudaGetLastError();
+    return launch_after(m.chained, bd ? kernb : kern, nblocks, NT, shmem, s, *m.x, *m.y, *m.a, *m.b,
+                        a, err, bd ? *bd : BatchDev{});
 }
 
 // Rows of a v band of a single simulation's tiles: the height for which the
@@ -754,9 +760,9 @@ static cudaError_t launch_any(const tma::StageMaps &m, const StageArgs &a, int s
 cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
                                  const CUtensorMap &mA, const CUtensorMap &mB, const StageArgs &a,
                                  int scheme, int stage, int fp32, int *err, int nblocks,
-                                 cudaStream_t s)
+                                 cudaStream_t s, bool chained)
 {
-    const tma::StageMaps m{&mX, &mY, &mA, &mB};
+    const tma::StageMaps m{&mX, &mY, &mA, &mB, chained};
     return launch_any(m, a, scheme, stage, fp32, err, nblocks, s, nullptr);
 }
 
@@ -764,23 +770,27 @@ cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
 // (scheme variant, precision); per-instance values come from bd.
 cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, int scheme,
                                        int stage, int fp32, int *err, int nblocks, int max_nvz,
-                                       cudaStream_t s)
+                                       cudaStream_t s, bool chained)
 {
     CUtensorMap z{};
-    const tma::StageMaps m{&z, &z, &z, &z};
+    const tma::StageMaps m{&z, &z, &z, &z, chained};
     return launch_any(m, a, scheme, stage, fp32, err, nblocks, s, &bd);
 }
 
-// Sets the shared-memory attribute of the kernels a simulation (or ensemble) of
-// this variant launches, on the current device.
-cudaError_t tma_prepare(int scheme, int fp32, bool gen)
+// Sets the shared-memory attribute of the kernels a simulation (batched: or an
+// ensemble) of this variant launches, on the current device.  The first call
+// loads them, 0.4 ms each.
+cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched)
 {
     CUtensorMap m{};
+    const BatchDev bd{};
+    const tma::StageMaps maps{&m, &m, &m, &m, false};
     StageArgs a{};
     a.fd_advec = gen;
     a.ko_order = 3;
     for (int st = 1; st <= 4; ++st) {
-        cudaError_t e = launch_rk4_stage_tma(m, m, m, m, a, scheme, st, fp32, nullptr, 0, nullptr);
+        cudaError_t e = launch_any(maps, a, scheme, st, fp32, nullptr, 0, nullptr,
+                                   batched ? &bd : nullptr);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -7,6 +7,7 @@
 
 #include <type_traits>
 
+#include "chain.cuh"
 #include "common.cuh"
 
 namespace cosenu {
@@ -156,8 +157,10 @@ template <bool INC, int STAGE> struct MapIdx {
 
 // The operand maps of one launch: X (stage input with halo), Y, A and B (see
 // the kernels' Layout; unused ones are ignored).
+// chained: the launch follows another stage launch of the same call (launch_after).
 struct StageMaps {
     const CUtensorMap *x, *y, *a, *b;
+    bool chained;
 };
 
 }  // namespace tma

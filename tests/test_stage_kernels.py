@@ -72,3 +72,29 @@ def test_fd_pipelined_kernel_edges(gpu_lib, oracle, nz, nvz, bc, fd_advec, ko, p
     case = Case(nz=nz, nvz=nvz, gz=4, z0=-nz / 4, z1=nz / 4, scheme="fd", bc=bc, omega=1e-2,
                 theta_deg=37.0, mat=True, mu=0.5, fd_advec=fd_advec, ko_order=ko)
     assert _compare(oracle, case, precision)[0] == 32
+
+
+# A call's launches overlap (a stage's blocks start before the previous stage has
+# ended); single-stage calls are launched one after the other.  Same bits, at one
+# tile, at less and more than a block per SM, and over a replayed step.
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("scheme", ["fv", "fd"])
+@pytest.mark.parametrize("nz,nvz", [(32, 8), (1000, 37), (9600, 40)])
+def test_overlapping_launches_keep_order(gpu_lib, oracle, nz, nvz, scheme, precision):
+    from oracle.oracle import Case
+    from tests._util import gpu_from_case
+    case = Case(nz=nz, nvz=nvz, gz=4, z0=-nz / 4, z1=nz / 4, scheme=scheme, omega=1e-2,
+                theta_deg=37.0, mu=0.5)
+    st0 = _rough(case, oracle, 1)
+    out = []
+    for overlap in (True, False):
+        with gpu_from_case(case, precision=precision) as sim:
+            sim.upload(st0)
+            if overlap:
+                for n in (1, 3, 19, 1):
+                    sim.evolve(n)
+            else:
+                for i in range(4 * 24):
+                    sim.step_stage(i % 4)
+            out.append(sim.download())
+    assert np.array_equal(*out)
