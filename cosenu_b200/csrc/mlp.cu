@@ -743,7 +743,7 @@ int cosenu_mlp_train(cosenu_mlp *net, int epochs, int batch, float lr, float wei
                 fa.scale = 1.f / ((float)rows * net->nout);
                 fa.loss = net->lossp + (size_t)(b0 / batch) * tiles;
                 fa.opt = opt;
-                MCK(mlptrain::step(fa, net->stream));
+                MCK(mlptrain::step(fa, net->stream, b0 > 0));
                 continue;
             }
             {

@@ -16,7 +16,9 @@
 // 512 x 512 weight gradient (64 columns: 8 and 32), and an operand's whole K is
 // staged at once (up to 128 x 576 x 2 B), so a GEMM is one round trip to L2, 4 MMAs
 // per 64 k behind it, and one commit.  2000 rows in batches of 64 (an epoch):
-// 6.85 -> 1.9 ms.
+// 6.85 -> 1.9 ms.  Launches overlap (chain.cuh): the next one's blocks start
+// when every tile has its accumulator, and allocate and wait behind the
+// epilogues.
 //
 // Every sum runs in the order of the separate kernels (k in steps of 16 within
 // one accumulator; bias gradients row by row), so the parameters a training
@@ -32,6 +34,7 @@
 #include <cstdint>
 #include <initializer_list>
 
+#include "chain.cuh"
 #include "mlp_math.cuh"
 #include "mlp_train.h"
 
@@ -150,7 +153,7 @@ struct Block8 {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             v[j] = (in && kg + j < ktot)
-                       ? __ldg(reinterpret_cast<const uint4 *>(X + (long long)(kg + j) * ld + rg))
+                       ? __ldcg(reinterpret_cast<const uint4 *>(X + (long long)(kg + j) * ld + rg))
                        : make_uint4(0, 0, 0, 0);
     }
     __device__ __forceinline__ void store(unsigned char *dst) const
@@ -346,14 +349,16 @@ __global__ void __launch_bounds__(NTHR) fwd_kernel(const __grid_constant__ Args 
     const int K = p.din[l], N = p.dout[l], n0 = blockIdx.x * TN, tid = threadIdx.x;
     const bool last = l == p.nl - 1;
     const int col = tid & (TN - 1), n = n0 + col;
-    const float bias = n < N ? p.w[p.boff[l] + n] : 0.f;
     Cta c(smem, rt, (K + 63) / 64, 1);
+    previous_launch();
+    const float bias = n < N ? p.w[p.boff[l] + n] : 0.f;
     const __nv_bfloat16 *X = l == 0 ? p.x : p.h[l - 1];
     float db = 0.f, loss = 0.f;
 #pragma unroll 1
     for (int m0 = 0; m0 < p.rows; m0 += rt) {
         if (last) copy_tile(c.tile, p.t, N, p.rows, N, m0, n0, rt);
         gemm_rows<false>(c, X, K, p.rows, K, p.wb + p.woff[l], K, N, m0, n0, rt, m0 == 0, p.err);
+        next_launch();
         c.spill();
 #pragma unroll 1
         for (int r = tid / TN; r < rt && m0 + r < p.rows; r += NTHR / TN) {
@@ -397,12 +402,14 @@ __device__ __forceinline__ void dx_tile(const Args &p, int l, int rt, int tile, 
     const int K = p.dout[l], N = p.din[l], n0 = tile * TN, tid = threadIdx.x;
     const int col = tid & (TN - 1);
     Cta c(smem, rt, (K + 63) / 64, 1);
+    previous_launch();
     float db = 0.f;
 #pragma unroll 1
     for (int m0 = 0; m0 < p.rows; m0 += rt) {
         copy_tile(c.tile, p.z[l - 1], N, p.rows, N, m0, n0, rt);
         gemm_rows<true>(c, p.dz[l], K, p.rows, K, p.wb + p.woff[l], N, N, m0, n0, rt, m0 == 0,
                         p.err);
+        next_launch();
         c.spill();
 #pragma unroll 1
         for (int r = tid / TN; r < rt && m0 + r < p.rows; r += NTHR / TN) {
@@ -425,6 +432,7 @@ __device__ __forceinline__ void dw_tile(const Args &p, int l, int tile, unsigned
     const int m0 = tile / nt * TM, n0 = tile % nt * TN, tid = threadIdx.x, col = tid & (TN - 1);
     const __nv_bfloat16 *X = l == 0 ? p.x : p.h[l - 1];
     Cta c(smem, TM, 1, 3);
+    previous_launch();
     const uint32_t la = lbo_a(TM);
     const size_t wo = p.woff[l];
     copy_tile(c.tile, p.w + wo, N, M, N, m0, n0, TM);
@@ -449,6 +457,7 @@ __device__ __forceinline__ void dw_tile(const Args &p, int l, int tile, unsigned
             mma_steps(c.tmem, su32(c.a), la, su32(c.b), 4, k0 == 0, su32(c.bar));
     }
     wait_copies();
+    next_launch();
     c.done(p.err);
     c.spill();
 #pragma unroll 2
@@ -509,22 +518,25 @@ cudaError_t prepare()
     return cudaSuccess;
 }
 
-cudaError_t step(const Args &a, cudaStream_t s)
+cudaError_t step(const Args &a, cudaStream_t s, bool chained)
 {
+    cudaError_t e = cudaSuccess;
     const int rt = tile_rows(a.rows), L = a.nl;
-    for (int l = 0; l < L; ++l)
-        fwd_kernel<<<(a.dout[l] + TN - 1) / TN, NTHR, smem_bytes(rt, k64(a.din[l]), 1), s>>>(a, l, rt);
+    for (int l = 0; l < L && e == cudaSuccess; ++l)
+        e = launch_after(chained || l > 0, fwd_kernel, (a.dout[l] + TN - 1) / TN, NTHR,
+                         smem_bytes(rt, k64(a.din[l]), 1), s, a, l, rt);
     auto dw_tiles = [&](int l) { return (a.dout[l] + TM - 1) / TM * (a.din[l] / TN); };
     const int dw_smem = smem_bytes(TM, 1, 3);
-    for (int l = L - 1; l >= 1; --l) {
+    for (int l = L - 1; l >= 1 && e == cudaSuccess; --l) {
         const int ndx = a.din[l] / TN, nw = l + 1 < L ? dw_tiles(l + 1) : 0;
         const int dx_smem = smem_bytes(rt, k64(a.dout[l]), 1);
-        bwd_kernel<<<ndx + nw, NTHR, dx_smem > dw_smem ? dx_smem : dw_smem, s>>>(a, l, ndx, l + 1,
-                                                                                nw, 0, rt);
+        e = launch_after(true, bwd_kernel, ndx + nw, NTHR, dx_smem > dw_smem ? dx_smem : dw_smem, s,
+                         a, l, ndx, l + 1, nw, 0, rt);
     }
     const int n1 = dw_tiles(1), n0 = dw_tiles(0);
-    bwd_kernel<<<n1 + n0, NTHR, dw_smem, s>>>(a, 0, 0, 1, n1, 0, rt);
-    return cudaGetLastError();
+    if (e == cudaSuccess)
+        e = launch_after(true, bwd_kernel, n1 + n0, NTHR, dw_smem, s, a, 0, 0, 1, n1, 0, rt);
+    return e;
 }
 
 }  // namespace mlptrain

@@ -36,7 +36,8 @@ bool fits(int nl, const int *din, const int *dout, int rows);
 int loss_tiles(int n_out);
 // Sets the kernels' shared-memory limit on the current device (before step).
 cudaError_t prepare();
-// Queues one training step on s.
-cudaError_t step(const Args &a, cudaStream_t s);
+// Queues one training step on s; chained: the previous operation there is a step
+// of the same call.
+cudaError_t step(const Args &a, cudaStream_t s, bool chained);
 
 }  // namespace mlptrain
