@@ -301,7 +301,7 @@ def run_ours(args):
             "gpu_launches": 4 * K,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": f"rk4_stage_tma_kernel<{sch}, stage {dom + 1}> "
+                         "kernel": f"rk4_stage_{'fv' if sch == 'FV' else 'tma'}_kernel<{sch}, stage {dom + 1}> "
                                    f"({sb[dom] // 64 if args.precision == 'fp64' else sb[dom]} "
                                    f"{'state passes' if args.precision == 'fp64' else 'B/cell'})",
                          "algorithmic_bytes_per_launch": algo_bytes,
