@@ -90,10 +90,13 @@ void choose_tile(cosenu_ctx *ctx, int layout = 0)
     const cosenu_params &p = ctx->p;
     const char *kenv = getenv("COSENU_KERNEL");
     bool force_ldg = kenv && std::string(kenv) == "ldg";
+    bool force_tma = kenv && std::string(kenv) == "tma";
     cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, p.device);
     const int nsm = ctx->nsm;
     // TMA path: every grid up to tma_max_nvz() rows (tiles are cut along v where
     // there are too few of them, and the last one of a row may be partial)
+    ctx->small = ctx->fp32 && p.scheme == FV && layout == 0 &&
+                 !(p.nz % 32 == 0 && (p.nz / 32 >= nsm || force_tma));
     const bool fits = p.nvz <= tma_max_nvz() && (p.nz % 32 == 0 || layout == 0);
     if (fits && (layout == 1 || (p.tile_z == 0 && p.tile_v == 0 && !force_ldg))) {
         ctx->use_tma = true;
@@ -135,7 +138,7 @@ StageArgs stage_args(const cosenu_ctx *ctx, int stage, int par)
     a.nvt = ctx->nvt;
     a.H = ctx->H;
     a.bc = ctx->p.bc;
-    a.flags = (int)ctx->p.flags;
+    a.flags = (int)ctx->p.flags | (ctx->small ? F_SMALL : 0);
     a.fd_advec = ctx->p.fd_advec;
     a.ko_order = ctx->p.ko_order;
     a.dt = ctx->dt;
@@ -519,7 +522,7 @@ int ctx_create(const cosenu_params *pp, cosenu_ctx **out, int layout)
             r = make_state_map(&ctx->mU2_40, ctx->U2, ub, ctx->ld, p.nvz, ctx->cs, bxu, rn);
         if (!ctx->U2) ctx->mU2_40 = ctx->mU1_40;  // unused in FP64
         if (!r && tma_prepare(p.scheme, ctx->fp32, p.fd_advec != 0 || p.ko_order == 5,
-                              layout == 1) != cudaSuccess)
+                              layout == 1, ctx->small) != cudaSuccess)
             r = -2;
         if (r) {
             // no tensor-map support: fall back to the register-tiled kernel

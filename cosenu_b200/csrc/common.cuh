@@ -24,7 +24,8 @@ constexpr int NMOM = 6;        // velocity moments per z
 
 enum Comp { EE = 0, XX, EXR, EXI, BEE, BXX, BEXR, BEXI };
 enum Scheme { FV = 0, FD = 1 };
-enum Flags { F_VAC = 1, F_MAT = 2, F_COLL = 4, F_ADVEC_OFF = 8 };
+// (F_SMALL: FP32-bulk FV on a small grid, see cosenu_ctx::small)
+enum Flags { F_VAC = 1, F_MAT = 2, F_COLL = 4, F_ADVEC_OFF = 8, F_SMALL = 1 << 16 };
 
 // Arguments of one RK4 stage launch (passed by value).
 struct StageArgs {

@@ -27,7 +27,7 @@ int tma_blocks_per_sm(int scheme);
 int fv_piece_rows(int nz, int nvz, int nsm);
 int fd_piece_rows(int nz, int nvz, int fp32, int nsm);
 int tma_blocks(int scheme, int nz, int nvt, int nsm);
-cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched);
+cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched, bool small);
 cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
                                  const CUtensorMap &mA, const CUtensorMap &mB, const StageArgs &a,
                                  int scheme, int stage, int fp32, int *err, int nblocks,
@@ -46,6 +46,10 @@ struct cosenu_ctx {
     long long cs = 0;
     double dz = 0, dv = 0, dt = 0, ct = 0, st = 0;
     int fp32 = 0;
+    // FP32-bulk FV adds the WENO candidates of a single simulation with less than
+    // one whole 32-cell tile per SM in another order (weno7_inc).  Its results
+    // have always differed from a large grid's by that rounding, and keep to it.
+    bool small = false;
     cudaStream_t own_stream = nullptr, stream = nullptr;
     // device memory.  Two FP64 state buffers Yb[0], Yb[1]: FP64 keeps the state
     // in Yb[0] and the RK4 accumulator in Yb[1]; FP32-bulk writes each step's

@@ -64,19 +64,19 @@ __device__ __forceinline__ double face_at(const TIN *__restrict__ X, const doubl
     if constexpr (INC) {
         // stencil differences as (Y difference in FP64, rounded) + (D
         // difference in FP32); the face is Y + (D + correction)
-        float dl[6];
+        float d[7];
         const double y0 = YPLUS ? ld_nc(Y + i) : (double)ld_nc(X + i);
         const float x0 = YPLUS ? (float)ld_nc(X + i) : 0.f;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const long long j0 = i + (k - 3) * dir, j1 = i + (k - 2) * dir;
+        for (int k = -3; k <= 3; ++k) {
+            if (k == 0) continue;
+            const long long j = i + k * dir;
             if constexpr (YPLUS)
-                dl[k] = (float)(ld_nc(Y + j1) - ld_nc(Y + j0)) +
-                        ((float)ld_nc(X + j1) - (float)ld_nc(X + j0));
+                d[k + 3] = (float)(ld_nc(Y + j) - y0) + ((float)ld_nc(X + j) - x0);
             else
-                dl[k] = (float)((double)ld_nc(X + j1) - (double)ld_nc(X + j0));
+                d[k + 3] = (float)((double)ld_nc(X + j) - y0);
         }
-        return y0 + (double)(x0 + weno7_corr12(dl) * (1.f / 12.f));
+        return y0 + (double)weno7_inc<false>(d[0], d[1], d[2], d[4], d[5], d[6], x0);
     } else {
         double u[7], dl[6];
 #pragma unroll

@@ -183,7 +183,8 @@ __device__ __forceinline__ Seg seg_of(const int4 e)
 // (FP64: U', U'' or Y; FP32-bulk: D1, D2, D3, then the new Y).  The
 // right-hand side is evaluated in FP64 in both forms, except the FP32-bulk
 // WENO7 weights and candidates (FP32 on FP64 stencil differences).
-template <int STAGE, class TIN, class TOUT, int NBUF, bool BATCHED, int MINB>
+// LARGE: the order of FP32-bulk's candidate sum (weno.cuh; FP64: true).
+template <int STAGE, class TIN, class TOUT, int NBUF, bool BATCHED, int MINB, bool LARGE>
 __global__ void __launch_bounds__(fv::NTHR, MINB)
     rk4_stage_fv_kernel(const __grid_constant__ CUtensorMap mX,
                         const __grid_constant__ CUtensorMap mY,
@@ -409,16 +410,13 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                     const TIN *x = xrow_of(r) + q * XW + je;
                     const double *y = yrow_of(r) + q * YW + je;
                     if constexpr (INC) {
-                        float dl[6];
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) {
-                            const int j1 = (k - 2) * s, j0 = (k - 3) * s;
-                            dl[k] = YPLUS ? (float)(y[j1] - y[j0]) + ((float)x[j1] - (float)x[j0])
-                                          : (float)((double)x[j1] - (double)x[j0]);
-                        }
-                        const float c = weno7_corr12(dl) * (1.f / 12.f);
-                        s_edge[b][r][q] = YPLUS ? y[0] + (double)((float)x[0] + c)
-                                                : (double)x[0] + (double)c;
+                        auto dif = [&](int n) {  // u(je + n s) - u(je)
+                            return YPLUS ? (float)(y[n * s] - y[0]) + ((float)x[n * s] - (float)x[0])
+                                         : (float)((double)x[n * s] - (double)x[0]);
+                        };
+                        const float f = weno7_inc<LARGE>(dif(-3), dif(-2), dif(-1), dif(1), dif(2),
+                                                         dif(3), YPLUS ? (float)x[0] : 0.f);
+                        s_edge[b][r][q] = (YPLUS ? y[0] : (double)x[0]) + (double)f;
                     } else {
                         double dl[6];
 #pragma unroll
@@ -434,7 +432,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                     const int q = 4 * p + qc;
                     double f[4];
                     if constexpr (INC) {
-                        float e[11], xs[12];
+                        float xs[12] = {0.f}, c[4];
                         double ys[12];
                         if constexpr (YPLUS) {
                             fv::load12(yrow + q * YW + qz - HALO, ys);
@@ -442,28 +440,13 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                         } else {
                             fv::load12(xrow + q * XW + qz - HALO, ys);
                         }
+                        auto dif = [&](int i, int j) {
+                            const float e = (float)(ys[j] - ys[i]);
+                            return YPLUS ? e + (xs[j] - xs[i]) : e;
+                        };
+                        weno7_inc_quad<LARGE>(dif, dir, xs + 4, c);
 #pragma unroll
-                        for (int k = 0; k < 11; ++k) {
-                            e[k] = (float)(ys[k + 1] - ys[k]);
-                            if (YPLUS) e[k] += xs[k + 1] - xs[k];
-                        }
-                        float dl[9], c[4];
-                        if (dir > 0) {
-#pragma unroll
-                            for (int k = 0; k < 9; ++k) dl[k] = e[k + 1];
-                            weno7_quad(dl, c);
-                        } else {
-                            float cr[4];
-#pragma unroll
-                            for (int k = 0; k < 9; ++k) dl[k] = e[9 - k];
-                            weno7_quad(dl, cr);
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) c[k] = -cr[3 - k];
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            f[k] = YPLUS ? ys[k + 4] + (double)(xs[k + 4] + c[k] * (1.f / 12.f))
-                                         : ys[k + 4] + (double)(c[k] * (1.f / 12.f));
+                        for (int k = 0; k < 4; ++k) f[k] = ys[k + 4] + (double)c[k];
                     } else {
                         double xs[12], dl[9], c[4];
                         fv::load12(xrow + q * XW + qz - HALO, xs);
@@ -724,8 +707,10 @@ template <int STAGE, class TIN, class TOUT, int NB, int MINB>
 static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *err, int nblocks,
                              cudaStream_t s, const BatchDev *bd)
 {
-    auto kern = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, false, MINB>;
-    auto kernb = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, true, MINB>;
+    constexpr bool INC = inc_form<TIN, TOUT>();
+    auto kern = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, false, MINB, true>;
+    auto kernb = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, true, MINB, true>;
+    if (INC && (a.flags & F_SMALL)) kern = rk4_stage_fv_kernel<STAGE, TIN, TOUT, NB, false, MINB, !INC>;
     if (nblocks <= 0) {  // preparation call: shared-memory limit and carveout (bd: both kernels)
         for (auto k : {kern, kernb}) {
             if (k == kernb && !bd) continue;

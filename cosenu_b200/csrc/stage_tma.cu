@@ -780,7 +780,7 @@ cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, i
 // Sets the shared-memory attribute of the kernels a simulation (batched: or an
 // ensemble) of this variant launches, on the current device.  The first call
 // loads them, 0.4 ms each.
-cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched)
+cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched, bool small)
 {
     CUtensorMap m{};
     const BatchDev bd{};
@@ -788,6 +788,7 @@ cudaError_t tma_prepare(int scheme, int fp32, bool gen, bool batched)
     StageArgs a{};
     a.fd_advec = gen;
     a.ko_order = 3;
+    a.flags = small ? F_SMALL : 0;
     for (int st = 1; st <= 4; ++st) {
         cudaError_t e = launch_any(maps, a, scheme, st, fp32, nullptr, 0, nullptr,
                                    batched ? &bd : nullptr);

@@ -30,27 +30,27 @@ namespace cosenu {
 // against 75 in the quadratic form, which shares nothing.
 constexpr double WENO_EPS = 1e-6 / 60.0;
 
-template <class T> struct WenoB {
-    T b0, b1, b2, b3;  // eps + beta_r, over 60
-    T Fa, Fb, Fc;      // fourth differences about centre + 1, centre, centre - 1
-    T q1;              // 12 x (candidate 1 - centre value)
+struct WenoB {
+    double b0, b1, b2, b3;  // eps + beta_r, over 60
+    double Fa, Fb, Fc;      // fourth differences about centre + 1, centre, centre - 1
+    double q1;              // 12 x (candidate 1 - centre value)
 };
 
-template <class T> __device__ __forceinline__ WenoB<T> weno7_indicators(const T *dl)
+__device__ __forceinline__ WenoB weno7_indicators(const double *dl)
 {
-    const T c13 = T(13.0 / 3.0), c781 = T(781.0 / 180.0), eps = T(WENO_EPS);
-    const T D0 = dl[1] - dl[0], D1 = dl[2] - dl[1], D2 = dl[3] - dl[2], D3 = dl[4] - dl[3],
+    const double c13 = 13.0 / 3.0, c781 = 781.0 / 180.0, eps = WENO_EPS;
+    const double D0 = dl[1] - dl[0], D1 = dl[2] - dl[1], D2 = dl[3] - dl[2], D3 = dl[4] - dl[3],
             D4 = dl[5] - dl[4];
-    const T T0 = D1 - D0, T1 = D2 - D1, T2 = D3 - D2, T3 = D4 - D3;
-    const T t0 = (c781 * T0) * T0 + eps, t1 = (c781 * T1) * T1 + eps, t2 = (c781 * T2) * T2 + eps,
+    const double T0 = D1 - D0, T1 = D2 - D1, T2 = D3 - D2, T3 = D4 - D3;
+    const double t0 = (c781 * T0) * T0 + eps, t1 = (c781 * T1) * T1 + eps, t2 = (c781 * T2) * T2 + eps,
             t3 = (c781 * T3) * T3 + eps;
-    const T C2 = dl[2] + dl[3];       // u[1] - u[-1]
-    const T dd = (c13 * D2) * D2;     // the inner sub-stencils' second difference
-    const T y1 = C2 - T(1.0 / 3.0) * T2, y2 = C2 - T(1.0 / 3.0) * T1;
-    const T e0 = D3 - T3, e3 = D1 + T0;  // the outer ones', continued to the centre
-    const T y0 = (T(2) * dl[3] - D3) + T(2.0 / 3.0) * T3;
-    const T y3 = (T(2) * dl[2] + D1) + T(2.0 / 3.0) * T0;
-    WenoB<T> r;
+    const double C2 = dl[2] + dl[3];       // u[1] - u[-1]
+    const double dd = (c13 * D2) * D2;     // the inner sub-stencils' second difference
+    const double y1 = C2 - (1.0 / 3.0) * T2, y2 = C2 - (1.0 / 3.0) * T1;
+    const double e0 = D3 - T3, e3 = D1 + T0;  // the outer ones', continued to the centre
+    const double y0 = (2. * dl[3] - D3) + (2.0 / 3.0) * T3;
+    const double y3 = (2. * dl[2] + D1) + (2.0 / 3.0) * T0;
+    WenoB r;
     r.b0 = (c13 * e0) * e0 + (y0 * y0 + t3);
     r.b1 = (y1 * y1 + dd) + t2;
     r.b2 = (y2 * y2 + dd) + t1;
@@ -58,7 +58,7 @@ template <class T> __device__ __forceinline__ WenoB<T> weno7_indicators(const T 
     r.Fc = T1 - T0;
     r.Fb = T2 - T1;
     r.Fa = T3 - T2;
-    r.q1 = T(6) * dl[3] + (dl[2] - dl[4]);
+    r.q1 = 6. * dl[3] + (dl[2] - dl[4]);
     return r;
 }
 
@@ -66,7 +66,7 @@ template <class T> __device__ __forceinline__ WenoB<T> weno7_indicators(const T 
 // centre + (q1 + num / den) / 12.
 __device__ __forceinline__ void weno7_parts(const double *dl, double &q1, double &num, double &den)
 {
-    const WenoB<double> r = weno7_indicators<double>(dl);
+    const WenoB r = weno7_indicators(dl);
     const double d0 = r.b0 * r.b0, d1 = r.b1 * r.b1, d2 = r.b2 * r.b2, d3 = r.b3 * r.b3;
     const double d01 = d0 * d1, d23 = d2 * d3;
     // gamma_r x prod_{k != r} d_k
@@ -113,23 +113,86 @@ __device__ __forceinline__ void weno7_quad(const double *dl, double *c12)
     for (int k = 0; k < 4; ++k) c12[k] = num[k] * inv[k] + q1[k];
 }
 
-// FP32-bulk form: 12 x (face - centre) in FP32 from differences the caller
-// takes in FP64, so that FP32 sees only the small differences and not the
-// O(1) values.  Same indicators and candidates; the weights use fast
+// FP32-bulk form: the face's increment, x0 + (face - centre), from the
+// stencil's differences to its centre, A .. G = u[-3..3] - u[0] (skipping the
+// centre), which the caller takes in FP64 so that FP32 sees only the small
+// differences and not the O(1) values; x0 is the centre's own increment.  The
+// indicators are the published quadratic forms; the weights use approximate
 // reciprocals (a common denominator would leave the FP32 range).
-__device__ __forceinline__ float weno7_corr12(const float *dl)
+//
+// The forms' cancellation is this option's largest error: on noise of 2e-2 a
+// face is within 1.2e-7, where the sums of squares above would give 8.5e-9.
+// FP32-bulk results are these roundings, though (sums of squares moved a state
+// by 6.5e-10 of its size in six rough steps), so every operation is written
+// out: the bits do not depend on what surrounds the call.  LARGE: whether
+// candidate 1 or 0 is the first product of the sum, the one that is rounded
+// before it is added.
+__device__ __forceinline__ float rcp_approx(float x)
 {
-    const WenoB<float> r = weno7_indicators<float>(dl);
-    const float w0 = __fdividef(4.f, r.b0 * r.b0), w1 = __fdividef(18.f, r.b1 * r.b1),
-                w2 = __fdividef(12.f, r.b2 * r.b2), w3 = __fdividef(1.f, r.b3 * r.b3);
-    const float num = w0 * r.Fa + w2 * r.Fb + w3 * (r.Fb - 3.f * r.Fc);
-    return r.q1 + __fdividef(num, (w0 + w1) + (w2 + w3));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-__device__ __forceinline__ void weno7_quad(const float *dl, float *c12)
+template <bool LARGE>
+__device__ __forceinline__ float weno7_inc(float A, float B, float Cc, float E, float F, float G,
+                                           float x0)
 {
+    // a x + b y + c z, and eps + P (..) + Q (..) + k R R
+    auto sum3 = [](float a, float x, float b, float y, float c, float z) {
+        return __fmaf_rn(c, z, __fmaf_rn(a, x, __fmul_rn(b, y)));
+    };
+    auto beta = [](float P, float p, float Q, float q, float k, float R) {
+        return __fadd_rn(1e-6f, __fmaf_rn(__fmul_rn(k, R), R, __fmaf_rn(P, p, __fmul_rn(Q, q))));
+    };
+    auto sum2 = [](float a, float x, float b, float y) { return __fmaf_rn(a, x, __fmul_rn(b, y)); };
+    const float b0 = beta(E, sum3(11003.f, E, -17246.f, F, 4642.f, G), F,
+                          sum2(7043.f, F, -3882.f, G), 547.f, G);
+    const float b1 = beta(Cc, sum3(547.f, Cc, 1922.f, E, -494.f, F), E,
+                          sum2(2843.f, E, -1642.f, F), 267.f, F);
+    const float b2 = beta(B, sum3(267.f, B, -1642.f, Cc, -494.f, E), Cc,
+                          sum2(2843.f, Cc, 1922.f, E), 547.f, E);
+    const float b3 = beta(A, sum3(547.f, A, -3882.f, B, 4642.f, Cc), B,
+                          sum2(7043.f, B, -17246.f, Cc), 11003.f, Cc);
+    // 12 x (candidate - centre)
+    const float q0 = __fadd_rn(__fmaf_rn(13.f, E, __fmul_rn(-5.f, F)), G);
+    const float q1 = __fsub_rn(__fmaf_rn(7.f, E, -Cc), F);
+    const float q2 = __fmaf_rn(3.f, E, __fmaf_rn(-5.f, Cc, B));
+    const float q3 = __fmaf_rn(-23.f, Cc, __fmaf_rn(13.f, B, __fmul_rn(-3.f, A)));
+    const float w0 = __fmul_rn(4.f, rcp_approx(__fmul_rn(b0, b0))),
+                w1 = __fmul_rn(18.f, rcp_approx(__fmul_rn(b1, b1))),
+                w2 = __fmul_rn(12.f, rcp_approx(__fmul_rn(b2, b2))),
+                w3 = rcp_approx(__fmul_rn(b3, b3));
+    const float n01 = LARGE ? __fmaf_rn(w1, q1, __fmul_rn(w0, q0))
+                            : __fmaf_rn(w0, q0, __fmul_rn(w1, q1));
+    const float num = __fmaf_rn(w3, q3, __fmaf_rn(w2, q2, n01));
+    const float sum = __fadd_rn(__fadd_rn(__fadd_rn(w0, w1), w2), w3);
+    return __fmaf_rn(num, rcp_approx(__fmul_rn(12.f, sum)), x0);
+}
+
+// The faces about cells 4 .. 7 of twelve, stencil direction dir: dif(i, j) is
+// u[j] - u[i] in FP32.  The differences between the four centres serve two faces
+// each (rounding is symmetric in sign).
+template <bool LARGE, class DIF>
+__device__ __forceinline__ void weno7_inc_quad(DIF dif, int dir, const float *x0, float *c)
+{
+    float in[4][4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c12[k] = weno7_corr12(dl + k);
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = i + 1; j < 4; ++j) {
+            in[i][j] = dif(i + 4, j + 4);
+            in[j][i] = -in[i][j];
+        }
+    auto d = [&](int k, int n) {  // u[k + n] - u[k]
+        return k + n >= 0 && k + n < 4 ? in[k][(k + n) & 3] : dif(k + 4, k + 4 + n);
+    };
+    const bool up = dir > 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float m3 = d(k, -3), m2 = d(k, -2), m1 = d(k, -1), p1 = d(k, 1), p2 = d(k, 2), p3 = d(k, 3);
+        c[k] = weno7_inc<LARGE>(up ? m3 : p3, up ? m2 : p2, up ? m1 : p1, up ? p1 : m1, up ? p2 : m2, up ? p3 : m3, x0[k]);
+    }
 }
 
 }  // namespace cosenu
