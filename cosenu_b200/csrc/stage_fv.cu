@@ -496,6 +496,10 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                     __syncwarp();
                 }
             } else {
+                // the edge warps arrive all the same, so that the barrier's phases
+                // follow the ring: an ensemble's block may go on to a member that
+                // advects
+                if (((warp - NE * ch) & (R - 1)) < NE) mbar_arrive(&ebar[b]);
 #pragma unroll
                 for (int q = 0; q < NCOMP; ++q) o[q] = 0.0;
             }
