@@ -97,6 +97,12 @@ int upload_args(cosenu_batch *b)
 // piece).
 int fv_pieces(const cosenu_batch *b, int i) { return ((b->m[i]->p.nvz + 7) / 8 + b->piece - 1) / b->piece; }
 
+// Rows of a piece of member i's tiles (FD: whole tiles).
+int tma_rows(const cosenu_batch *b, int i)
+{
+    return b->scheme == COSENU_FV ? 8 * b->piece : b->m[i]->p.nvz;
+}
+
 // Table of the work of the members in `active`, member by member.  TMA family,
 // FD: one entry per z tile, `ranges` splitting the table into at most max_blk
 // contiguous runs of equal work.  TMA family, FV: one entry per piece of a z
@@ -277,7 +283,8 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
 int apply_tiling(cosenu_batch *b)
 {
     for (int i = 0; i < b->n; ++i) {
-        int rc = b->use_tma ? ctx_set_tiling(b->m[i], 0, 0) : ctx_set_tiling(b->m[i], b->tz, b->tv[i]);
+        int rc = b->use_tma ? ctx_set_tiling(b->m[i], 0, tma_rows(b, i))
+                            : ctx_set_tiling(b->m[i], b->tz, b->tv[i]);
         if (rc) return bfail(b, rc, cosenu_last_error(b->m[i]));
     }
     return upload_args(b);
@@ -349,6 +356,9 @@ int cosenu_batch_create(int n, const cosenu_params *params, cosenu_batch **out)
         }
         if (pc == max_piece) b->piece = piece;
     }
+    for (int i = 0; i < n; ++i)
+        if (b->m[i]->use_tma && ctx_set_tiling(b->m[i], 0, tma_rows(b, i)) != COSENU_OK)
+            return bail(COSENU_ERR_ARG);
     if (cudaMalloc(&b->d_args, 8 * (size_t)n * sizeof(StageArgs)) != cudaSuccess ||
         cudaMalloc(&b->d_maps, 2 * NMAP_B * (size_t)n * sizeof(CUtensorMap)) != cudaSuccess ||
         cudaMalloc(&b->err_flag, 64) != cudaSuccess)

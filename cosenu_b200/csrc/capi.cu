@@ -557,20 +557,13 @@ int ctx_normalise_parity(cosenu_ctx *ctx)
 
 int ctx_set_tiling(cosenu_ctx *ctx, int tz, int tv)
 {
-    if (tz == 0) {
-        ctx->tz = 32;
-        ctx->tv = ctx->p.nvz;
-        ctx->nvt = 1;
-        ctx->use_tma = true;
-    } else {
-        int nvt = (ctx->p.nvz + tv - 1) / tv;
-        if (ctx->p.nz % tz != 0 || nvt > ctx->mom_nvt_cap || tv > MAX_TV)
-            return fail(ctx, COSENU_ERR_ARG, "tile does not fit this member");
-        ctx->tz = tz;
-        ctx->tv = tv;
-        ctx->nvt = nvt;
-        ctx->use_tma = false;
-    }
+    const int nvt = (ctx->p.nvz + tv - 1) / tv;
+    if (nvt > ctx->mom_nvt_cap || (tz != 0 && (ctx->p.nz % tz != 0 || tv > MAX_TV)))
+        return fail(ctx, COSENU_ERR_ARG, "tile does not fit this member");
+    ctx->tz = tz == 0 ? 32 : tz;
+    ctx->tv = tv;
+    ctx->nvt = nvt;
+    ctx->use_tma = tz == 0;
     drop_graphs(ctx);
     return ctx->have_state ? prepare_state(ctx) : COSENU_OK;
 }
@@ -1005,7 +998,7 @@ int cosenu_tile(const cosenu_ctx *ctx, int *tile_z, int *tile_v)
 {
     if (!ctx) return COSENU_ERR_ARG;
     if (tile_z) *tile_z = ctx->tz;
-    if (tile_v) *tile_v = ctx->tv;
+    if (tile_v) *tile_v = std::min(ctx->tv, ctx->p.nvz);
     return COSENU_OK;
 }
 

@@ -109,6 +109,8 @@ int ctx_normalise_parity(cosenu_ctx *ctx);
 void ctx_flip(cosenu_ctx *ctx);
 // Ghost cells and input moments of Y after Y changed outside the stages.
 int ctx_prepare_state(cosenu_ctx *ctx);
-// Re-tiles an ensemble member for the register-tiled kernel (tz x tv) or back
-// to the TMA layout (tz = 0); recomputes the input moments of Y.
+// Re-tiles an ensemble member for the register-tiled kernel (tz x tv) or for the
+// TMA layout (tz = 0, tiles in pieces of tv rows); recomputes the input moments
+// of Y.  The member's own launches and the ensemble's hand each other the moments
+// of Y, so both cut a tile alike.
 int ctx_set_tiling(cosenu_ctx *ctx, int tz, int tv);

@@ -164,7 +164,7 @@ __device__ __forceinline__ Seg seg_of(int i, const StageArgs &a, int nzt)
     s.piece = i / nzt;
     s.zt = i - s.piece * nzt;
     s.np = a.nvt;
-    const int pc = a.tv / R;
+    const int pc = (a.tv + R - 1) / R;
     s.c0 = s.piece * pc;
     s.c1 = min(s.c0 + pc, (a.nvz + R - 1) / R);
     return s;

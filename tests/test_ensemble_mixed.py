@@ -66,3 +66,38 @@ def test_members_with_and_without_advection(gpu_lib, monkeypatch, precision):
     for i, x in enumerate(xs):
         want = _alone(x, i, precision, x.nsteps, monkeypatch)
         assert np.abs(got[i] - want).max() <= TOL[precision], i
+
+
+# The shared launches and a member's own read each other's moments of the state.
+# Step by step, as a stretch and stage by stage between two shared runs; row counts
+# that are and are not multiples of the 8-row chunk, and fewer rows than one.
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("scheme", ["fv", "fd"])
+@pytest.mark.parametrize("tiled", [False, True])
+def test_members_step_on_their_own_between_runs(gpu_lib, monkeypatch, scheme, precision, tiled):
+    from cosenu_b200.ensemble import Ensemble
+    xs = [_member(nz, nvz, 0) for nz, nvz in ((256, 37), (512, 64), (96, 5), (4736, 24))]
+    with Ensemble(xs, scheme=scheme, precision=precision) as ens:
+        if tiled:
+            ens.set_config(False, 16, [16, 24, 5, 8])
+        for i, (x, m) in enumerate(zip(xs, ens.members)):
+            m.upload(_rough(x, i))
+        ens.run([2, 3, 1, 2])
+        for m in ens.members:
+            m.step_rk4()
+            m.evolve(2)
+            for s in range(4):
+                m.step_stage(s)
+        ens.run([1, 2, 2, 1])
+        ens.synchronize()
+        got = [m.download() for m in ens.members]
+    from cosenu_b200 import NuOsc
+    monkeypatch.setenv("COSENU_KERNEL", "tma")
+    for i, (x, n) in enumerate(zip(xs, (7, 9, 7, 7))):
+        p = x.params(scheme, precision)
+        if tiled:
+            p.tile_z, p.tile_v = 16, (16, 24, 5, 8)[i]
+        with NuOsc(p) as sim:
+            sim.upload(_rough(x, i))
+            sim.evolve(n)
+            assert np.abs(got[i] - sim.download()).max() <= 3 * TOL[precision], i
