@@ -318,6 +318,14 @@ int copy_planes_h2d(cosenu_ctx *ctx, double *dst, const double *const *src, int 
 
 void drop_graphs(cosenu_ctx *ctx)
 {
+    // a captured step that was not replayed often enough to pay for its capture:
+    // single steps wait twice as long for the next one, so that a program which
+    // changes a parameter every few steps stops capturing (600 x 32 FV cells, mu set
+    // every 1 / 10 / 50 steps: 254 / 50 / 30 us a step capturing after eight single
+    // steps each time, 32 / 26 / 26 so, and as without graphs)
+    if (ctx->singles >= ctx->single_min && (ctx->g1[0] || ctx->g1[1]) && ctx->replays < 64)
+        ctx->single_min = std::min(2 * ctx->single_min, 1 << 20);
+    ctx->singles = ctx->replays = 0;
     for (int k = 0; k < 2; ++k) {
         if (ctx->g1[k]) cudaGraphExecDestroy(ctx->g1[k]);
         if (ctx->gN[k]) cudaGraphExecDestroy(ctx->gN[k]);
@@ -810,15 +818,17 @@ int cosenu_step(cosenu_ctx *ctx, int nsteps)
     if (nsteps == 0) return COSENU_OK;
     DeviceGuard dg(ctx->p.device);
     // A program that calls for one step at a time gets the captured step from its
-    // ninth call on (one launch instead of four: 600 x 32 FV cells, 32.8 -> 26.6 us a
-    // call); a capture costs as much as a few dozen launches.  Not inside a
+    // ninth call on (one launch instead of four: 600 x 32 FV cells, 26.5 -> 24.6 us a
+    // call, 34.3 -> 30.2 with a synchronisation behind it); a capture costs 0.22 ms,
+    // so it is put off further where it did not pay (drop_graphs).  Not inside a
     // capture of the caller's own.
     bool direct = !ctx->use_graphs;
     if (nsteps == 1 && !direct) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         CK(cudaStreamIsCapturing(ctx->stream, &cap));
         direct = cap != cudaStreamCaptureStatusNone ||
-                 (!ctx->g1[ctx->ypar] && ctx->singles < 8 && ++ctx->singles);
+                 (!ctx->g1[ctx->ypar] && ctx->singles < ctx->single_min && ++ctx->singles);
+        if (!direct && ctx->replays < 64) ++ctx->replays;
     }
     if (direct) {
         CK(launch_steps(ctx, nsteps, ctx->stream));

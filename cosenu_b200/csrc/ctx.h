@@ -78,7 +78,9 @@ struct cosenu_ctx {
     // graphs of 1 and GRAPH_CHUNK steps, per parity of the state buffer
     cudaGraphExec_t g1[2] = {nullptr, nullptr}, gN[2] = {nullptr, nullptr};
     bool use_graphs = true;
-    int singles = 0;  // calls for a single step launched directly
+    // calls for a single step since the graphs were last dropped: those launched
+    // directly, at most single_min, then replays of the captured step
+    int singles = 0, single_min = 8, replays = 0;
     // status
     bool have_state = false, have_profile = false, have_state0 = false;
     int next_stage = 0;
