@@ -84,33 +84,34 @@ __device__ __forceinline__ double weno7_corr12(const double *dl)
     return q1 + num / den;
 }
 
-// 1 / D0 .. 1 / D3 from one division: the product of the four, its
-// reciprocal, then products of the others.  Denominators of weno7_parts lie
-// in [7e-46, 1e21] where the stencil differences are at most 2 in magnitude
-// (density-matrix entries of O(1)), so the product of four stays far inside
-// the FP64 range.
-__device__ __forceinline__ void recip4(double D0, double D1, double D2, double D3, double &i0,
-                                       double &i1, double &i2, double &i3)
-{
-    const double p01 = D0 * D1, p23 = D2 * D3;
-    const double r = 1.0 / (p01 * p23);
-    const double r01 = r * p23, r23 = r * p01;
-    i0 = r01 * D1;
-    i1 = r01 * D0;
-    i2 = r23 * D3;
-    i3 = r23 * D2;
-}
-
 // 12 x (face - centre) of four consecutive faces from the nine differences of
-// their ten cells.
+// their ten cells, with one division: the reciprocal of the product of the four
+// denominators, times the others.
+//
+// Denominators lie in [7e-46, 1e21] where the stencil differences are at most 2
+// in magnitude (density-matrix entries of O(1)), so the product of four is far
+// inside the FP64 range.  States in other units leave it (differences of 1e5 and
+// more); then, and for non-finite cells, every face has its own division.
 __device__ __forceinline__ void weno7_quad(const double *dl, double *c12)
 {
-    double q1[4], num[4], den[4], inv[4];
+    double q1[4], num[4], den[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) weno7_parts(dl + k, q1[k], num[k], den[k]);
-    recip4(den[0], den[1], den[2], den[3], inv[0], inv[1], inv[2], inv[3]);
+    const double p01 = den[0] * den[1], p23 = den[2] * den[3], p = p01 * p23;
+    // (denominators are positive: their high words order as the values do)
+    const unsigned top = max(max((unsigned)__double2hiint(p01), (unsigned)__double2hiint(p23)),
+                             (unsigned)__double2hiint(p));
+    if (top < 0x7fb00000u) {  // 2^1020: the reciprocals are normal numbers
+        const double r = 1.0 / p;
+        const double r01 = r * p23, r23 = r * p01;
+        c12[0] = num[0] * (r01 * den[1]) + q1[0];
+        c12[1] = num[1] * (r01 * den[0]) + q1[1];
+        c12[2] = num[2] * (r23 * den[3]) + q1[2];
+        c12[3] = num[3] * (r23 * den[2]) + q1[3];
+    } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c12[k] = num[k] * inv[k] + q1[k];
+        for (int k = 0; k < 4; ++k) c12[k] = q1[k] + num[k] / den[k];
+    }
 }
 
 // FP32-bulk form: the face's increment, x0 + (face - centre), from the
