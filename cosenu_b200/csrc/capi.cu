@@ -1008,7 +1008,7 @@ int cosenu_tile(const cosenu_ctx *ctx, int *tile_z, int *tile_v)
 {
     if (!ctx) return COSENU_ERR_ARG;
     if (tile_z) *tile_z = ctx->tz;
-    if (tile_v) *tile_v = std::min(ctx->tv, ctx->p.nvz);
+    if (tile_v) *tile_v = ctx->use_tma ? std::min(ctx->tv, ctx->p.nvz) : ctx->tv;
     return COSENU_OK;
 }
 
