@@ -83,7 +83,7 @@ __device__ __forceinline__ double face_at(const TIN *__restrict__ X, const doubl
         for (int k = -3; k <= 3; ++k) u[k + 3] = in_at<YPLUS>(X, Y, i + k * dir);
 #pragma unroll
         for (int k = 0; k < 6; ++k) dl[k] = u[k + 1] - u[k];
-        return u[3] + weno7_corr12(dl) * (1.0 / 12.0);
+        return __fma_rn(weno7_corr12(dl), 1.0 / 12.0, u[3]);
     }
 }
 

@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
 #pragma unroll
                         for (int k = 0; k < 6; ++k)
                             dl[k] = (double)x[(k - 2) * s] - (double)x[(k - 3) * s];
-                        s_edge[b][r][q] = (double)x[0] + weno7_corr12(dl) * (1.0 / 12.0);
+                        s_edge[b][r][q] = __fma_rn(weno7_corr12(dl), 1.0 / 12.0, (double)x[0]);
                     }
                     mbar_arrive(&ebar[b]);
                 }
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(fv::NTHR, MINB)
                             for (int k = 0; k < 4; ++k) c[k] = cr[3 - k];
                         }
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) f[k] = xs[k + 4] + c[k] * (1.0 / 12.0);
+                        for (int k = 0; k < 4; ++k) f[k] = __fma_rn(c[k], 1.0 / 12.0, (double)xs[k + 4]);
                     }
                     double *w = s_face[warp];
                     *reinterpret_cast<double2 *>(w + fv::face_at(qc, qz)) = make_double2(f[0], f[1]);
