@@ -233,8 +233,9 @@ struct cosenu_mlp {
     size_t nparam = 0;
     float *w = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // FP32 flat
     __nv_bfloat16 *wb = nullptr;                                      // BF16 copy (flat)
-    // activations for up to `cap` rows
+    // activations for up to `cap` rows, one allocation
     int cap = 0;
+    void *act = nullptr;
     __nv_bfloat16 *xb = nullptr;
     std::vector<float *> Z;           // pre-activations [cap][dout]
     std::vector<__nv_bfloat16 *> Hb;  // activations [cap][dout]
@@ -243,12 +244,12 @@ struct cosenu_mlp {
     float *T = nullptr, *partial = nullptr;  // partial: 1024 floats, then eacc
     double *eacc = nullptr;                   // epoch loss sum, on the device
     // fused training: gradients per layer, an epoch's rows in shuffled order,
-    // loss partials of every step
+    // loss partials of every step, one allocation
     std::vector<__nv_bfloat16 *> dz;
-    int dz_cap = 0;
     __nv_bfloat16 *xe = nullptr;
     float *te = nullptr, *lossp = nullptr;
-    size_t xe_cap = 0, te_cap = 0, lossp_cap = 0;
+    void *fus = nullptr;
+    size_t fus_bytes = 0;
     // resident training data
     float *dX = nullptr, *dT = nullptr;
     int *didx = nullptr;
@@ -371,61 +372,73 @@ int stage_inputs(cosenu_mlp *net, const float *x_host, const float *t_host, int 
     return COSENU_OK;
 }
 
+// Cuts arrays out of one allocation (256-byte aligned); sizes only while base is
+// null.  A free is a device synchronisation, so a network that is made, trained
+// briefly and dropped pays for every array it holds.
+struct Arena {
+    char *base;
+    size_t used = 0;
+    template <class T> void take(T *&p, size_t n)
+    {
+        p = reinterpret_cast<T *>(base + used);
+        used += (n * sizeof(T) + 255) / 256 * 256;
+    }
+};
+
 int ensure_cap(cosenu_mlp *net, int rows)
 {
     if (rows <= net->cap) return COSENU_OK;
     cudaStreamSynchronize(net->stream);
-    auto fr = [](void *p) { if (p) cudaFree(p); };
-    fr(net->xb);
-    for (auto p : net->Z) fr(p);
-    for (auto p : net->Hb) fr(p);
-    fr(net->dA); fr(net->dB); fr(net->dAb); fr(net->T);
-    int wmax = std::max(net->kpad, std::max(net->nh, net->nout));
-    MCK(cudaMalloc(&net->xb, (size_t)rows * net->kpad * 2));
-    for (int l = 0; l < net->nl; ++l) {
-        MCK(cudaMalloc(&net->Z[l], (size_t)rows * net->dout[l] * 4));
-        MCK(cudaMalloc(&net->Hb[l], (size_t)rows * net->dout[l] * 2));
-    }
-    MCK(cudaMalloc(&net->dA, (size_t)rows * wmax * 4));
-    MCK(cudaMalloc(&net->dB, (size_t)rows * wmax * 4));
-    MCK(cudaMalloc(&net->dAb, (size_t)rows * wmax * 2));
-    MCK(cudaMalloc(&net->T, (size_t)rows * net->nout * 4));
+    if (net->act) cudaFree(net->act);
+    net->act = nullptr;
+    net->cap = 0;
+    const size_t wmax = std::max(net->kpad, std::max(net->nh, net->nout)), n = rows;
+    auto cut = [&](Arena a) {
+        a.take(net->xb, n * net->kpad);
+        for (int l = 0; l < net->nl; ++l) {
+            a.take(net->Z[l], n * net->dout[l]);
+            a.take(net->Hb[l], n * net->dout[l]);
+        }
+        a.take(net->dA, n * wmax);
+        a.take(net->dB, n * wmax);
+        a.take(net->dAb, n * wmax);
+        a.take(net->T, n * net->nout);
+        return a.used;
+    };
+    MCK(cudaMalloc(&net->act, cut(Arena{nullptr})));
+    cut(Arena{static_cast<char *>(net->act)});
     net->cap = rows;
     return COSENU_OK;
 }
 
 // Buffers of the fused training path: `batch` rows per step, ndata rows and
-// nsteps steps per epoch.
-int ensure_fused(cosenu_mlp *net, int batch, int nsteps)
+// nsteps steps per epoch.  False where device memory has no room for them: the
+// separate launches need none, and give the same parameters.
+bool ensure_fused(cosenu_mlp *net, int batch, int nsteps)
 {
-    auto grow = [&](void **p, size_t &cap, size_t n) -> int {
-        if (n <= cap) return COSENU_OK;
-        cudaStreamSynchronize(net->stream);
-        if (*p) cudaFree(*p);
-        *p = nullptr;
-        cap = 0;
-        MCK(cudaMalloc(p, n));
-        cap = n;
-        return COSENU_OK;
+    const size_t nd = net->ndata;
+    auto cut = [&](Arena a) {
+        for (int l = 0; l < net->nl; ++l) a.take(net->dz[l], (size_t)batch * net->dout[l]);
+        a.take(net->xe, nd * net->kpad);
+        a.take(net->te, nd * net->nout);
+        a.take(net->lossp, (size_t)nsteps * mlptrain::loss_tiles(net->nout));
+        return a.used;
     };
-    int rc;
-    if ((rc = grow((void **)&net->xe, net->xe_cap, (size_t)net->ndata * net->kpad * 2)) ||
-        (rc = grow((void **)&net->te, net->te_cap, (size_t)net->ndata * net->nout * 4)) ||
-        (rc = grow((void **)&net->lossp, net->lossp_cap,
-                   (size_t)nsteps * mlptrain::loss_tiles(net->nout) * 4)))
-        return rc;
-    if (batch > net->dz_cap) {
+    net->dz.resize(net->nl);
+    const size_t need = cut(Arena{nullptr});
+    if (need > net->fus_bytes) {
         cudaStreamSynchronize(net->stream);
-        for (auto &p : net->dz) {
-            if (p) cudaFree(p);
-            p = nullptr;
+        if (net->fus) cudaFree(net->fus);
+        net->fus = nullptr;
+        net->fus_bytes = 0;
+        if (cudaMalloc(&net->fus, need) != cudaSuccess) {
+            cudaGetLastError();  // (not an error of this call)
+            return false;
         }
-        net->dz_cap = 0;
-        net->dz.resize(net->nl, nullptr);
-        for (int l = 0; l < net->nl; ++l) MCK(cudaMalloc(&net->dz[l], (size_t)batch * net->dout[l] * 2));
-        net->dz_cap = batch;
+        net->fus_bytes = need;
     }
-    return COSENU_OK;
+    cut(Arena{static_cast<char *>(net->fus)});
+    return true;
 }
 
 // forward over `rows` rows already in net->xb; output pre-activation of the
@@ -555,17 +568,10 @@ int cosenu_mlp_destroy(cosenu_mlp *net)
 {
     if (!net) return COSENU_OK;
     if (net->stream) cudaStreamSynchronize(net->stream);
-    void *bufs[] = {net->w, net->g, net->m1, net->m2, net->wb, net->partial, net->xb, net->dA,
-                    net->dB, net->dAb, net->T, net->dX, net->dT, net->didx, net->dxin, net->dtin,
-                    net->derr, net->xe, net->te, net->lossp};
+    void *bufs[] = {net->w, net->g, net->m1, net->m2, net->wb, net->partial, net->act, net->fus,
+                    net->dX, net->dT, net->didx, net->dxin, net->dtin, net->derr};
     for (void *b : bufs)
         if (b) cudaFree(b);
-    for (auto p : net->Z)
-        if (p) cudaFree(p);
-    for (auto p : net->Hb)
-        if (p) cudaFree(p);
-    for (auto p : net->dz)
-        if (p) cudaFree(p);
     collect_times(net);
     for (cudaEvent_t e : net->ev_pool) cudaEventDestroy(e);
     if (net->stream) cudaStreamDestroy(net->stream);
@@ -691,11 +697,11 @@ int cosenu_mlp_train(cosenu_mlp *net, int epochs, int batch, float lr, float wei
     // timing mode needs the separate launches it brackets by class.
     const int nsteps = (net->ndata + batch - 1) / batch, tiles = mlptrain::loss_tiles(net->nout);
     const bool fused = net->tc && !net->timing &&
-                       mlptrain::fits(net->nl, net->din.data(), net->dout.data(), batch);
+                       mlptrain::fits(net->nl, net->din.data(), net->dout.data(), batch) &&
+                       ensure_fused(net, batch, nsteps);
     std::vector<float> lossp;
     mlptrain::Args fa{};
     if (fused) {
-        if ((rc = ensure_fused(net, batch, nsteps)) != COSENU_OK) return rc;
         MCK(mlptrain::prepare());
         lossp.resize((size_t)nsteps * tiles);
         fa.nl = net->nl;
