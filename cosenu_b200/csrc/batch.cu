@@ -161,16 +161,11 @@ size_t build_table(cosenu_batch *b, const std::vector<int> &active, std::vector<
     std::vector<std::pair<long long, int4>> t;
     for (int i : active) {
         const cosenu_params &p = b->m[i]->p;
-        if (b->use_tma) {
-            for (int zt = 0; zt < p.nz / 32; ++zt)
-                t.push_back({(long long)p.nvz * 32, make_int4(i, zt, 0, 0)});
-        } else {
-            const int tv = b->tv[i], nvt = (p.nvz + tv - 1) / tv;
-            for (int vt = 0; vt < nvt; ++vt)
-                for (int zt = 0; zt < p.nz / b->tz; ++zt)
-                    t.push_back({(long long)std::min(tv, p.nvz - vt * tv) * b->tz,
-                                 make_int4(i, zt, vt, 0)});
-        }
+        const int tv = b->tv[i], nvt = (p.nvz + tv - 1) / tv;
+        for (int vt = 0; vt < nvt; ++vt)
+            for (int zt = 0; zt < p.nz / b->tz; ++zt)
+                t.push_back({(long long)std::min(tv, p.nvz - vt * tv) * b->tz,
+                             make_int4(i, zt, vt, 0)});
     }
     std::stable_sort(t.begin(), t.end(),
                      [](const std::pair<long long, int4> &x, const std::pair<long long, int4> &y) {
@@ -217,8 +212,6 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
     BatchDev bd0{b->d_table[k], (int)nt, b->d_args, b->d_maps,
                  reinterpret_cast<const int *>(b->d_table[k] + nt)};
     if (b->scheme == COSENU_FD && getenv("COSENU_BATCH_RR")) bd0.range = nullptr;
-    int max_nvz = 0;
-    for (int i : active) max_nvz = std::max(max_nvz, b->m[i]->p.nvz);
     const StageArgs a0 = ctx_stage_args(b->m[active[0]], 1);
     // the active members' common buffer parity (0 for FP64)
     int par = b->m[active[0]]->ypar;
@@ -230,7 +223,7 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
             cudaError_t e;
             if (b->use_tma)
                 e = launch_rk4_stage_tma_batch(bd, a0, b->scheme, st, b->fp32, b->err_flag, nblk,
-                                               max_nvz, s, chained || st > 1);
+                                               s, chained || st > 1);
             else
                 e = launch_rk4_stage_batch(bd, b->scheme, st, b->tz, b->fp32, s);
             if (e != cudaSuccess) return e;
@@ -239,9 +232,12 @@ int run_phase(cosenu_batch *b, const std::vector<int> &active, long long nsteps)
     };
     // Long phases: one graph of 16 steps, replayed (an even number, so that every
     // replay starts from the same parity).  Short ones are launched directly: a
-    // capture costs about 0.5 ms of host time, as much as 45 steps of four
-    // launches, and held up runs of many short phases (16 members, 14 phases of a
-    // few steps: 7 of 10 ms).
+    // capture costs 0.3 to 0.5 ms of host time and held up runs of many short phases
+    // (16 members, 14 phases of a few steps: 7 of 10 ms).  Phases of 16 / 64 / 96 /
+    // 160 steps, us, direct against graph: two 256 x 16 FV members 474 / 1842 / 2747
+    // / - and 741 / 1828 / 2502 / 3958, FD 455 / 1778 / 2659 / - and 741 / 2031 /
+    // 2883 / 4607; 16 members of 512-4096 cells the same from 64 steps on.  Small FV
+    // members gain from 64 steps on, small FD ones lose to beyond 96.
     const int chunk = 16;
     cudaGraphExec_t ge = nullptr;
     if (nsteps >= 8 * chunk) {
@@ -341,7 +337,9 @@ int cosenu_batch_create(int n, const cosenu_params *params, cosenu_batch **out)
     }
     // FV: the piece height (chunks) for which dealing all members' entries out
     // over the block slots takes the fewest chunk times, at a third of a chunk of
-    // overhead per entry
+    // overhead per entry.  us a step by height, [chosen]: 16 members of 512-4096
+    // cells 1 1144, 2 902, 3 875, [4] 817, 6 865, 8 826, 16 905; the first four of
+    // them 1 214, [2] 187, 3 204, 4 194, 8 234
     double best = 1e300;
     const long long slots = (long long)tma_blocks_per_sm(b->scheme) * b->nsm;
     const int max_piece = (b->max_nvz + 7) / 8;
@@ -519,7 +517,7 @@ int cosenu_batch_autotune(cosenu_batch *b, int trial_steps, char *report, size_t
         if (apply_tiling(b) != COSENU_OK) return 1e30f;
         for (int i = 0; i < b->n; ++i)
             if (ctx_normalise_parity(b->m[i]) != COSENU_OK) return 1e30f;
-        if (run_phase(b, all, 1) != COSENU_OK) return 1e30f;  // warm-up (graph capture)
+        if (run_phase(b, all, 1) != COSENU_OK) return 1e30f;  // warm-up
         cudaEventRecord(e0, b->stream);
         if (run_phase(b, all, trial_steps) != COSENU_OK) return 1e30f;
         cudaEventRecord(e1, b->stream);

@@ -52,13 +52,13 @@ struct StageArgs {
 // Ensemble launch: one stage launch covers every active instance.  Entry t of
 // `table` names (instance, z tile, v tile, -) in the register-tiled family,
 // (instance, z tile, -, rows) in FD's TMA kernel and (instance, z tile, chunks,
-// moment pieces) in FV's (stage_fv.cu); `args` holds the four stage arguments of every instance and `maps` its six tensor maps (Y and U0/U1
-// input boxes; Y, A and U0 tile boxes).
+// moment pieces) in FV's (stage_fv.cu); `args` holds the four stage arguments of
+// every instance and `maps` its eight tensor maps (tma.cuh: MapIdx).
 struct BatchDev {
     const int4 *table;
     int ntiles;
     const StageArgs *args;      // [instances][4]
-    const CUtensorMap *maps;    // [instances][5]
+    const CUtensorMap *maps;    // [instances][8]
     const int *range;           // TMA family: block b owns table entries [range[b], range[b+1])
 };
 

@@ -33,7 +33,7 @@ cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
                                  int scheme, int stage, int fp32, int *err, int nblocks,
                                  cudaStream_t s, bool chained);
 cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, int scheme,
-                                       int stage, int fp32, int *err, int nblocks, int max_nvz,
+                                       int stage, int fp32, int *err, int nblocks,
                                        cudaStream_t s, bool chained);
 cudaError_t launch_rk4_stage_batch(const BatchDev &bd, int scheme, int stage, int tz, int fp32,
                                    cudaStream_t s);

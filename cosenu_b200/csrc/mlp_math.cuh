@@ -1,10 +1,6 @@
 // Elementwise pieces of the surrogate network shared by its kernels.
 #pragma once
 
-#include <cuda_bf16.h>
-
-#include <cstdint>
-
 namespace mlpmath {
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
@@ -33,12 +29,6 @@ __device__ __forceinline__ void adamw(float &w, float &m, float &v, float gi, co
     const float mh = mi / p.c1, vh = vi / p.c2;
     const float u = mh / (sqrtf(vh) + p.eps);
     w = __fmaf_rn(-p.lr, __fmaf_rn(wd, w, u), w);
-}
-
-__device__ __forceinline__ uint32_t pack2(float lo, float hi)
-{
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(lo)) |
-           ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(hi)) << 16);
 }
 
 }  // namespace mlpmath

@@ -688,7 +688,11 @@ int fv_box_x(int elem_bytes) { return elem_bytes == 8 ? fv::xw<double>() : fv::x
 
 // Rows of a v piece of a single simulation's tiles: the height (a multiple of
 // 8) for which the rounds of items over the block slots take the fewest
-// chunk times, at half a chunk of overhead per item.
+// chunk times, at half a chunk of overhead per item.  us a step by height in chunks,
+// [chosen]: 600 x 32 [1] 21.9, 2 31.6, 4 54.1; 1024 x 64 [1] 28.1, 2 33.1, 4 53.9;
+// 2400 x 100 1 79.8, [2] 77.5, 4 81.6; 9600 x 64 1 183, [2] 165, 4 171; 4000 x 100 2
+// 114, 5 113, [7] 116, 13 149; 16384 x 64 1 308, 2 267, [8] 274.  It misses 2400 x 32
+// (1 37.3, [2] 42.4: 300 chunks on 296 slots) and 8192 x 128 (3 260, [16] 284).
 int fv_piece_rows(int nz, int nvz, int nsm)
 {
     const int nzt = (nz + tma::TZ - 1) / tma::TZ, nch = (nvz + fv::R - 1) / fv::R;

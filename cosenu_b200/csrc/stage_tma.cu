@@ -634,7 +634,10 @@ static cudaError_t launch_nb(const tma::StageMaps &m, const StageArgs &a, int *e
 
 // Rows of a v band of a single simulation's tiles: the height for which the
 // rounds of items over the SMs take the fewest chunk times, summed over the four
-// stages, at one chunk of overhead per item.
+// stages, at one chunk of overhead per item.  us a step by height, [chosen]: 1000 x
+// 37 8 20.1, [12] 17.1, 16 19.1, 32 27.1; 2000 x 64 16 30.0, [32] 27.1, 64 43.5;
+// 4000 x 100 16 78, 32 72, 64 66.4, [100] 67.0; 8192 x 128 32 174, 64 176, [128]
+// 168; 16384 x 64 16 202, [32] 175, 64 172.
 int fd_piece_rows(int nz, int nvz, int fp32, int nsm)
 {
     const int nzt = (nz + tma::TZ - 1) / tma::TZ;
@@ -769,7 +772,7 @@ cudaError_t launch_rk4_stage_tma(const CUtensorMap &mX, const CUtensorMap &mY,
 // Ensemble launch: `a` carries the variant switches shared by every instance
 // (scheme variant, precision); per-instance values come from bd.
 cudaError_t launch_rk4_stage_tma_batch(const BatchDev &bd, const StageArgs &a, int scheme,
-                                       int stage, int fp32, int *err, int nblocks, int max_nvz,
+                                       int stage, int fp32, int *err, int nblocks,
                                        cudaStream_t s, bool chained)
 {
     CUtensorMap z{};

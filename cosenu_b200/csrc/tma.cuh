@@ -146,8 +146,8 @@ __device__ __forceinline__ void fence_proxy_async_smem()
 // FP64:      0 Y (halo box), 1 U0 (halo), 2 U1 (halo), 3 Y (tile), 4 A (tile), 5 U0 (tile)
 // FP32-bulk: 0 current Y (halo), 1 D1 (halo), 2 D2 (halo), 3 D2 (tile), 5 D1 (tile), 6 D3 (halo),
 //            7 current Y (halo) in the row count of stage 4
-// (FV launches read U0 at FP64 stage 3 and D1, D2 at FP32-bulk stage 4 with
-// plain loads instead.)
+// (FV launches copy U0 at FP64 stage 3 and D1, D2 at FP32-bulk stage 4 row by row,
+// without a map.)
 template <bool INC, int STAGE> struct MapIdx {
     static constexpr int X = STAGE == 1 ? 0 : (STAGE == 3 ? 2 : (INC && STAGE == 4 ? 6 : 1));
     static constexpr int Y = INC ? (STAGE == 4 ? 7 : 0) : 3;
