@@ -52,7 +52,7 @@ struct StageArgs {
 // Ensemble launch: one stage launch covers every active instance.  Entry t of
 // `table` names (instance, z tile, v tile, -) in the register-tiled family,
 // (instance, z tile, -, rows) in FD's TMA kernel and (instance, z tile, chunks,
-// moment pieces) in FV's (stage_fv.cu); `args` holds the four stage arguments of
+// moment pieces) in FV's (stage_fv.cuh); `args` holds the four stage arguments of
 // every instance and `maps` its eight tensor maps (tma.cuh: MapIdx).
 struct BatchDev {
     const int4 *table;

@@ -1,5 +1,5 @@
 // TMA-pipelined RK4 stage kernel of the FD scheme (src/rhs_fd.hpp:6-148); the
-// FV scheme's is stage_fv.cu.
+// FV scheme's is stage_fv.cuh.
 //
 // Same arithmetic and epilogue as rk4_stage_kernel (stage.cu); what changes
 // is how the operands reach the SM.  Each block is persistent over work items:

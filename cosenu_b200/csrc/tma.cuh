@@ -1,5 +1,5 @@
 // Shared pieces of the TMA-pipelined stage kernels (stage_tma.cu: FD,
-// stage_fv.cu: FV): bounded mbarrier waits, tensor-map copies, ensemble table
+// stage_fv.cuh: FV): bounded mbarrier waits, tensor-map copies, ensemble table
 // helpers and the launch interface.
 #pragma once
 
@@ -233,9 +233,12 @@ inline int tma_smem_limit(int minb)
     return minb == 1 ? TMA_SMEM_MAX : TMA_SMEM_SM / minb - 1024;
 }
 
-// FV launches (stage_fv.cu); nblocks <= 0: sets the kernels' attributes.
+// FV launches (stage_fv.cu, FP32-bulk's in stage_fv32.cu); nblocks <= 0: sets the
+// kernels' attributes.
 cudaError_t launch_fv_tma(const tma::StageMaps &m, const StageArgs &a, int stage, int fp32, int *err,
                           int nblocks, cudaStream_t s, const BatchDev *bd);
+cudaError_t launch_fv_bulk(const tma::StageMaps &m, const StageArgs &a, int stage, int *err,
+                           int nblocks, cudaStream_t s, const BatchDev *bd);
 int fv_blocks_per_sm();
 int fv_box_x(int elem_bytes);
 
