@@ -1,8 +1,8 @@
 """FP32-bulk FV results are their FP32 roundings: the WENO indicators' cancellation
 moves a face by up to 1e-7 of the stencil's differences, so another form of them,
 or another order of a sum, is another result (2e-8 here).  The states are held to
-what the register-tiled (small grids) and the pipelined kernel gave when the
-option came in (commit 9cacf60), three steps from rough data.
+what the register-tiled (small grids) and the pipelined kernel gave at commit
+9cacf60, three steps from rough data.
 
 Tolerance: FP64 sums may be ordered differently (1e-13), and where that turns one
 FP32 rounding of an increment of at most 0.05 over, a cell moves by 6e-8 x 0.05 =
